@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                                                                   Vert* __restrict__ verts, size_t n_slots,
                                                                   float* __restrict__ inv_wsum_px, WorkCounters* wc) {
     extern __shared__ int smem_raw[];
-    int* stack = smem_raw + threadIdx.x;
+    int* stack = lane_stack(smem_raw);
     const int lane = threadIdx.x & 31;
     uint32_t err = 0;
     const uint32_t n_st = R.s_end - R.s_begin;
@@ -634,13 +634,13 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
             }
             if (!__any_sync(kFullMask, state != A_IDLE)) break;
             const size_t slot = slot_base + (size_t)(cur - R.s_begin) * 32;
-            if (state == A_CLOSEST || state == A_SHADOW) {
-                const bool shadow = state == A_SHADOW;
+            {
+                const bool shadow = state == A_SHADOW, act = shadow || state == A_CLOSEST;
                 Ray r;
                 r.o = P.ray.o;
                 r.d = shadow ? pend.dir : P.ray.d;
                 r.time = shadow ? 0.0f : P.ray.time;
-                if (!walking) {
+                if (act && !walking) {
                     h.t = shadow ? pend.tmax : CUDART_INF_F;
                     h.prim = -1;
                     h.b1 = h.b2 = 0.0f;
@@ -648,10 +648,10 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                     tv.sp = 0;
                     found = false;
                 }
-                walking = !trace_resume<false, false, LUM_SUSPEND_LANES, CLS>(S, r, 0.001f, shadow, h, found, tv, stack,
-                                                                             err);
-                if (walking) {
-                    // suspended: resumes in a later iteration
+                walking = !walk_warp<false, false, LUM_SUSPEND_LANES, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err,
+                                                                          act) && act;
+                if (walking || !act) {
+                    // no walk, or suspended: resumes in a later iteration
                 } else if (shadow) {
                     if (!found) {
                         P.L = P.L + pend.contrib;
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                     state = P.bounce >= R.max_depth ? A_DONE : A_CLOSEST;
                 } else if (!found) {
                     bg = background(S, R, P.ray);                     // render.rs:1535
-                    P.L = P.L + mul(P.beta, bg);
+                    add_light(P, bg);
                     state = A_DONE;
                 } else {
                     const Ray in = P.ray;
@@ -834,7 +834,7 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
         int nsm = 0, devi = 0;
         cudaGetDevice(&devi);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, devi);
-        const size_t stack = (size_t)kStackDepth * 128 * sizeof(int);
+        const size_t stack = stack_smem(kStackDepth, 128);
         auto replay = dev.cls == CLS_QUAD ? adj::k_replay<CLS_QUAD>
                     : dev.cls == CLS_MESH ? adj::k_replay<CLS_MESH> : adj::k_replay<CLS_ALL>;
         int occ_r = 0;

@@ -31,10 +31,13 @@ __global__ void __launch_bounds__(kAovThreads) k_aov(SceneDev S, RenderDev R, fl
                                                      uint8_t* __restrict__ normals, uint8_t* __restrict__ albedo,
                                                      WorkCounters* wc) {
     extern __shared__ int s_stack[];
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     uint32_t err = 0;
     const size_t n = (size_t)R.w * R.h;
-    for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
+    // warps go on together: a lane past the end walks along without a ray
+    for (size_t w0 = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < n; w0 += (size_t)gridDim.x * blockDim.x) {
+        const bool act = w0 + (threadIdx.x & 31u) < n;
+        const size_t o = act ? w0 + (threadIdx.x & 31u) : w0;
         const uint32_t i = (uint32_t)(o % R.w), j = (uint32_t)(o / R.w);
         const uint32_t gi = i + R.crop_x, gj = j + R.crop_y;
         const uint32_t pixel = gj * R.full_w + gi;
@@ -46,7 +49,9 @@ __global__ void __launch_bounds__(kAovThreads) k_aov(SceneDev S, RenderDev R, fl
         h.b1 = h.b2 = 0.0f;
         float dv = 0.0f;
         uint8_t nb[3] = {0, 0, 0}, ab[3] = {0, 0, 0};
-        if (trace<false>(S, P.ray, 0.001f, false, h, stack, err)) {
+        const bool found = trace<false>(S, P.ray, 0.001f, false, h, stack, err, act);
+        if (!act) continue;
+        if (found) {
             dv = h.t;
             const Surface sf = surface_of(S, P.ray, h);
             nb[0] = clamp_byte((sf.n.x * 0.5f + 0.5f) * 255.0f);
@@ -84,7 +89,7 @@ __global__ void __launch_bounds__(kAovThreads) k_aov(SceneDev S, RenderDev R, fl
 
 cudaError_t launch_aov(const SceneDev& S, const RenderDev& R, float* depth, uint8_t* normals, uint8_t* albedo,
                        WorkCounters* wc, cudaStream_t stream) {
-    const size_t stack = (size_t)kStackDepth * kAovThreads * sizeof(int);
+    const size_t stack = stack_smem(kStackDepth, kAovThreads);
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_aov, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stack);

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kRenderThreads, SPH ? (NEE ? 6 : 7) : CLS != C
     __shared__ unsigned long long s_acc[kRenderThreads / 32][32][4];
     __shared__ uint32_t s_next[kRenderThreads / 32];
     __shared__ V s_exit[kRenderThreads / 32][32];      // deferred Subsurface origins (EXT only)
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t err = 0, nseg = 0, nsh = 0;
     TestTally tally{};
@@ -182,10 +182,14 @@ __device__ void hit_uv(const SceneDev& S, const Ray& ray, const Hit& h, const Su
 __global__ void __launch_bounds__(kRenderThreads) k_intersect(SceneDev S, const lum_ray* __restrict__ rays, uint32_t n,
                                                               lum_hit* __restrict__ hits, WorkCounters* wc) {
     extern __shared__ int s_stack[];
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     uint32_t err = 0;
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        lum_ray r = rays[idx];
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    // warps go on together: a lane past the end walks along without a ray
+    for (uint64_t w0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < n; w0 += stride) {
+        const uint64_t idx = w0 + (threadIdx.x & 31u);
+        const bool act = idx < n;
+        lum_ray r = rays[act ? idx : w0];
         Ray ray{mk(r.org), mk(r.dir), r.time};
         Hit h;
         h.t = r.tmax;
@@ -193,7 +197,9 @@ __global__ void __launch_bounds__(kRenderThreads) k_intersect(SceneDev S, const 
         h.b1 = h.b2 = 0.0f;
         lum_hit out;
         out.reserved = 0;
-        if (trace(S, ray, r.tmin, false, h, stack, err)) {
+        const bool found = trace(S, ray, r.tmin, false, h, stack, err, act);
+        if (!act) continue;
+        if (found) {
             Surface sf = surface_of(S, ray, h);
             out.t = h.t;
             hit_uv(S, ray, h, sf, out.u, out.v);
@@ -219,15 +225,19 @@ __global__ void __launch_bounds__(kRenderThreads) k_intersect(SceneDev S, const 
 __global__ void __launch_bounds__(kRenderThreads) k_occluded(SceneDev S, const lum_ray* __restrict__ rays, uint32_t n,
                                                              int32_t* __restrict__ occ, WorkCounters* wc) {
     extern __shared__ int s_stack[];
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     uint32_t err = 0;
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        lum_ray r = rays[idx];
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t w0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < n; w0 += stride) {
+        const uint64_t idx = w0 + (threadIdx.x & 31u);
+        const bool act = idx < n;
+        lum_ray r = rays[act ? idx : w0];
         Ray ray{mk(r.org), mk(r.dir), r.time};
         Hit h;
         h.t = r.tmax;
         h.prim = -1;
-        occ[idx] = trace(S, ray, r.tmin, true, h, stack, err) ? 1 : 0;
+        const bool found = trace(S, ray, r.tmin, true, h, stack, err, act);
+        if (act) occ[idx] = found ? 1 : 0;
     }
     if (err) atomicOr(&wc->error_flags, err);
 }
@@ -243,7 +253,7 @@ static int num_sms() {
     return n;
 }
 
-static size_t stack_bytes(int threads) { return (size_t)kStackDepth * threads * sizeof(int); }
+static size_t stack_bytes(int threads) { return stack_smem(kStackDepth, threads); }
 
 static int render_occupancy() {
     static const int occ = [] {   // initialised once, thread-safe
@@ -389,7 +399,7 @@ static cudaError_t launch_render_t(const SceneDev& S, const RenderDev& R, float*
                                          : k_render<COUNT, false, COUNT, false, CLS_MESH>)
                         : (nee ? k_render<COUNT, false, true, false> : k_render<COUNT, false, COUNT, false>);
     // the traversal stack sized to the scene's BVH; resident blocks for that size
-    const size_t smem = (size_t)S.stack_depth * kRenderThreads * sizeof(int);
+    const size_t smem = stack_smem(S.stack_depth, kRenderThreads);
     if (blocks_per_sm == occ) blocks_per_sm = kernel_occupancy((const void*)kernel, smem);
     int grid = num_sms() * blocks_per_sm;
     int blocks_needed = (int)((n_total + 3) / 4);   // 4 warps per block, one task per warp at least

@@ -48,21 +48,21 @@ __device__ __forceinline__ void fixed_pixel(const unsigned long long* a, float e
     for (int c = 0; c < 3; ++c) o[c] = (float)((double)(long long)a[c] / kFixScale * inv) * exposure;
 }
 
-// One lane's traversal and shading step (state ST_CLOSEST or ST_SHADOW): the closest hit of its
-// path segment or the any hit of its NEE shadow ray, walked (or resumed) through the same code,
-// then the shading step once the walk is complete.  A walk suspended by trace_resume leaves the
-// state unchanged and resumes in a later iteration.
+// The warp's traversal and shading step: for a lane in state ST_CLOSEST or ST_SHADOW the closest hit
+// of its path segment or the any hit of its NEE shadow ray, walked (or resumed) through the same
+// code, then its shading step once the walk is complete.  A walk suspended by walk_warp leaves
+// the state unchanged and resumes in a later iteration.  Called by all 32 lanes.
 template <bool COUNT, bool EXT, bool NEE, bool SPH, int SUSPEND, int CLS>
 __device__ __forceinline__ void path_step(const SceneDev& S, const RenderDev& R, uint32_t pixel, int& state, Path& P,
                                           Pending& pend, Hit& h, Trav& tv, bool& found, bool& walking, V* stash,
                                           int* stack, uint32_t& err, uint32_t& nseg, uint32_t& nsh,
                                           TestTally* tally) {
-    const bool shadow = state == ST_SHADOW;
+    const bool shadow = state == ST_SHADOW, act = shadow || state == ST_CLOSEST;
     Ray r;
     r.o = P.ray.o;
     r.d = shadow ? pend.dir : P.ray.d;
     r.time = shadow ? 0.0f : P.ray.time;                      // Ray::new (render.rs:1457)
-    if (!walking) {
+    if (act && !walking) {
         h.t = shadow ? (EXT ? fabsf(pend.tmax) : pend.tmax) : CUDART_INF_F;
         h.prim = -1;
         h.b1 = h.b2 = 0.0f;
@@ -70,8 +70,8 @@ __device__ __forceinline__ void path_step(const SceneDev& S, const RenderDev& R,
         tv.sp = 0;
         found = false;
     }
-    walking = !trace_resume<COUNT, SPH, SUSPEND, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err, tally);
-    if (walking) return;
+    walking = !walk_warp<COUNT, SPH, SUSPEND, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err, act, tally) && act;
+    if (walking || !act) return;
     if (shadow) {
         ++nsh;
         if (!found) P.L = P.L + pend.contrib;
@@ -120,9 +120,8 @@ __device__ __forceinline__ void tile_task(const SceneDev& S, const RenderDev& R,
             }
         }
         if (!__any_sync(full, state != ST_IDLE)) break;
-        if (state == ST_CLOSEST || state == ST_SHADOW)
-            path_step<COUNT, EXT, NEE, SPH, SUSPEND, CLS>(S, R, pixel, state, P, pend, h, tv, found, walking,
-                                                          exit_stash + lane, stack, err, nseg, nsh, tally);
+        path_step<COUNT, EXT, NEE, SPH, SUSPEND, CLS>(S, R, pixel, state, P, pend, h, tv, found, walking,
+                                                      exit_stash + lane, stack, err, nseg, nsh, tally);
         if (state == ST_DONE) {
             const float4 v = path_sample(R, P.L, P.jx, P.jy);
             add_fixed(&acc[cur][0], v.x);

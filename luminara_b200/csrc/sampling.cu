@@ -83,33 +83,8 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
             }
         }
         if (!__any_sync(kAll, state != ST_IDLE)) break;
-        if (state == ST_CLOSEST || state == ST_SHADOW) {
-            const bool shadow = state == ST_SHADOW;
-            Ray r;
-            r.o = P.ray.o;
-            r.d = shadow ? pend.dir : P.ray.d;
-            r.time = shadow ? 0.0f : P.ray.time;                  // Ray::new (render.rs:1457)
-            if (!walking) {
-                h.t = shadow ? (EXT ? fabsf(pend.tmax) : pend.tmax) : CUDART_INF_F;
-                h.prim = -1;
-                h.b1 = h.b2 = 0.0f;
-                tv.node = S.n_nodes > 0 ? 0 : kSentinel;
-                tv.sp = 0;
-                found = false;
-            }
-            walking = !trace_resume<false, SPH, LUM_SUSPEND_LANES>(S, r, 0.001f, shadow, h, found, tv, stack, err);
-            if (walking) {
-                // suspended: resumes in a later iteration
-            } else if (shadow) {
-                ++nsh;
-                if (!found) P.L = P.L + pend.contrib;
-                shadow_done<EXT>(P, pend, exit_stash + lane);
-                state = P.bounce >= R.max_depth ? ST_DONE : ST_CLOSEST;
-            } else {
-                ++nseg;
-                state = shade<-1, EXT, NEE, SPH>(S, R, pixel, P, found, h, pend, exit_stash + lane);
-            }
-        }
+        path_step<false, EXT, NEE, SPH, LUM_SUSPEND_LANES, CLS_ALL>(S, R, pixel, state, P, pend, h, tv, found, walking,
+                                                                   exit_stash + lane, stack, err, nseg, nsh, nullptr);
         if (state == ST_DONE) {
             if (acc) {
                 const float4 v = path_sample(R, P.L, P.jx, P.jy);
@@ -140,7 +115,7 @@ __global__ void __launch_bounds__(kSampThreads, ADAPTIVE ? 4 : 5) k_render_sampl
     __shared__ uint32_t s_slot[kSampWarps][32];
     __shared__ uint32_t s_next[kSampWarps];
     __shared__ V s_exit[kSampWarps][32];            // deferred Subsurface origins
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t err = 0, nseg = 0, nsh = 0;
     unsigned long long kept = 0;
@@ -238,7 +213,7 @@ template <bool ADAPTIVE, bool EXT, bool NEE, bool SPH>
 cudaError_t launch_t(const SceneDev& S, const RenderDev& R, const SamplingDev& A, float* out, WorkCounters* wc,
                      cudaStream_t stream) {
     // the traversal stack sized to the scene's BVH; resident blocks per stack size (cached)
-    const size_t stack = (size_t)S.stack_depth * kSampThreads * sizeof(int);
+    const size_t stack = stack_smem(S.stack_depth, kSampThreads);
     static std::mutex mu;
     static bool attr = false;
     static std::vector<std::pair<size_t, int>> occ_of;
@@ -247,7 +222,7 @@ cudaError_t launch_t(const SceneDev& S, const RenderDev& R, const SamplingDev& A
         std::lock_guard<std::mutex> lk(mu);
         if (!attr) {
             cudaFuncSetAttribute(k_render_sampled<ADAPTIVE, EXT, NEE, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)((size_t)kStackDepth * kSampThreads * sizeof(int)));
+                                 (int)stack_smem(kStackDepth, kSampThreads));
             attr = true;
         }
         for (const auto& e : occ_of)

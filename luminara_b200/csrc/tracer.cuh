@@ -367,125 +367,171 @@ __device__ __forceinline__ bool hit_plane(const PlaneDev& P, const Ray& ray, flo
 
 // ------------------------------------------------------------------------------ traversal
 // BVH2 traversal with postponed leaves (the "while-while" organisation of Aila & Laine,
-// "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009): a lane that reaches a
-// leaf keeps it pending and goes on descending inner nodes until every active lane of the
-// warp holds a leaf; then all lanes test their leaves together.  Inner nodes are visited
+// "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009), one warp at a time: the
+// whole warp runs the two loops below in step, every lane with a walk visiting inner nodes until
+// each of them holds a leaf, then all lanes testing their leaves together.  Inner nodes are visited
 // near child first.  Stack entries (shared memory, entry k of thread j at
 // stack[k * blockDim.x + j]) are inner-node indices (>= 0) or leaf ranges ~(first << 3 |
-// count - 1); kSentinel marks the empty stack.
+// count - 1); entry 0 holds kSentinel, so a pop needs no test for the empty stack.
 constexpr int kSentinel = 0x7fffffff;
 
-// Place of a suspended BVH walk (trace_resume): the next node to visit (an inner node index, or
-// kSentinel when the walk is over) and the stack depth; the stack entries stay in shared memory
-// and the closest hit so far in the caller's Hit.
+// Bytes of dynamic shared memory of a block's stacks of `depth` entries (and the sentinel).
+__host__ __device__ constexpr size_t stack_smem(int depth, int threads) {
+    return (size_t)(depth + 1) * threads * sizeof(int);
+}
+// The thread's stack in the block's dynamic shared memory, its sentinel set.
+__device__ __forceinline__ int* lane_stack(int* smem) {
+    int* s = smem + threadIdx.x;
+    *s = kSentinel;
+    return s;
+}
+
+// Shared-memory accesses (32-bit addresses) under a predicate rather than a branch: the lanes of
+// a visit that pop and those that push stay together.
+__device__ __forceinline__ void load_if(bool p, uint32_t addr, int& v) {
+    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\n@q ld.shared.b32 %0, [%1];\n}"
+                 : "+r"(v) : "r"(addr), "r"((int)p) : "memory");
+}
+__device__ __forceinline__ void store_if(bool p, uint32_t addr, int v) {
+    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\n@q st.shared.b32 [%0], %1;\n}"
+                 :: "r"(addr), "r"(v), "r"((int)p) : "memory");
+}
+
+// Two f32 fused multiply-adds in one instruction (each rounded as fmaf rounds).
+__device__ __forceinline__ unsigned long long pair_of(float x) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float2 fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+    float2 r;
+    asm("{\n.reg .b64 t;\nfma.rn.f32x2 t, %2, %3, %4;\nmov.b64 {%0, %1}, t;\n}"
+        : "=f"(r.x), "=f"(r.y) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Place of a suspended BVH walk (walk_warp): the next node to visit (an inner node index, or
+// kSentinel when the walk is over) and the stack's depth in bytes; the stack entries stay in
+// shared memory and the closest hit so far in the caller's Hit.
 struct Trav {
     int node;
     int sp;
 };
 
-// The BVH walk of `trace`, resumable.  With SUSPEND > 0 the walk stops at the top of an outer
-// iteration (no postponed leaf pending) once at most SUSPEND lanes of the warp are still
-// walking: it saves its place in tv and returns false, so that the lanes which finished can
-// shade and start new rays before the warp walks on (Aila & Laine 2009 replace terminated rays
-// in the same spirit: a warp's traversal otherwise runs as long as its longest ray while the
-// finished lanes idle).  Returns true when the walk is complete (planes tested, `found` final).
-// SUSPEND == 0 never stops early.  tv starts as {0, 0} (or kSentinel for a scene without
-// nodes), found as false.
+// The BVH walks of a warp, resumable.  Called by all 32 lanes; `act`: the lane has a walk (its
+// place in tv, {0, 0} at the start, or kSentinel for a scene without nodes; found as false).
+// With SUSPEND > 0 the call returns once at most SUSPEND lanes are still walking (none of them
+// holding a leaf): those keep their place in tv, so that the lanes which finished can shade and
+// start new rays before the warp walks on (Aila & Laine 2009 replace terminated rays in the same
+// spirit: a warp's traversal otherwise runs as long as its longest ray while the finished lanes
+// idle).  Returns true for a lane whose walk is complete (planes tested, `found` final).
+//
+// What bounds it is instruction issue and how many lanes each instruction serves.  So both loops
+// are the warp's: their conditions are full-warp votes, which also bring the lanes together
+// after every visit and every primitive test; the stack is moved by predicated accesses; a leaf's
+// primitives and a second pending leaf follow each other in one loop, so a lane with a short
+// leaf takes its next one meanwhile; and the slab tests use the packed f32 FMA.  The earlier form
+// (each lane's own loops, which the compiler let diverge: 11.4 lanes per instruction on the box
+// room, 7.2 on the mixed scenes) against this one, same box, same images: sphere field 1080p 64
+// spp 23.0 -> 21.8 ms, dense mesh 1080p 16 spp 20.2 -> 17.8, quads 512x512 9.77 -> 8.56, box room
+// 1.99 -> 1.83, twelve mixed scenes 236 -> 200, adaptive sphere field 34.4 -> 30.7.
+// Leaving the node loop once at most 3 lanes lack a leaf gained 1-2% on the sphere field and the
+// mesh and lost 7-9% on the room and the materials' scene; leaving it only when no lane can
+// walk on (no vote on leaves) lost 4-13%; leaving the leaf loop with 2, 6 or 12 lanes' leaves
+// unfinished lost 2-10%; branches instead of the predicated accesses lost up to 3%.
 template <bool COUNT = false, bool SPH = false, int SUSPEND = 0, int CLS = CLS_ALL>
-__device__ __forceinline__ bool trace_resume(const SceneDev& S, const Ray& ray, float tmin, bool any, Hit& hit,
-                                             bool& found, Trav& tv, int* stack, uint32_t& err,
-                                             TestTally* tl = nullptr) {
-    if (tv.node != kSentinel) {
-        // Reciprocals of direction components clamped away from zero: the FMA slab form
-        // lo*inv - o*inv would give inf - inf = NaN for an axis-parallel ray, while a finite
-        // +-1e20 keeps the ordering of the reference's (lo - o) * (1/d) (aabb.rs:23-25).
-        const float ix = 1.0f / (fabsf(ray.d.x) > 1e-20f ? ray.d.x : copysignf(1e-20f, ray.d.x));
-        const float iy = 1.0f / (fabsf(ray.d.y) > 1e-20f ? ray.d.y : copysignf(1e-20f, ray.d.y));
-        const float iz = 1.0f / (fabsf(ray.d.z) > 1e-20f ? ray.d.z : copysignf(1e-20f, ray.d.z));
-        const float ox = -ray.o.x * ix, oy = -ray.o.y * iy, oz = -ray.o.z * iz;
-        // the sphere class divides by |d|^2 once per walk instead of once per sphere test
-        float ia_ray = 0.0f;
-        if constexpr (SPH && !COUNT) ia_ray = 1.0f / len2(ray.d);
-        const float4* nodes = reinterpret_cast<const float4*>(S.nodes);
-        const int stride = blockDim.x;
-        int sp = tv.sp;
-        int node = tv.node;   // inner node index, leaf (< 0) or kSentinel
-        int leaf = 0;         // postponed leaf (< 0) or 0
+__device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, float tmin, bool any, Hit& hit,
+                                          bool& found, Trav& tv, int* stack, uint32_t& err, bool act,
+                                          TestTally* tl = nullptr) {
+    constexpr unsigned full = 0xffffffffu;
+    // Reciprocals of direction components clamped away from zero: the FMA slab form
+    // lo*inv - o*inv would give inf - inf = NaN for an axis-parallel ray, while a finite
+    // +-1e20 keeps the ordering of the reference's (lo - o) * (1/d) (aabb.rs:23-25).
+    const float ix = 1.0f / (fabsf(ray.d.x) > 1e-20f ? ray.d.x : copysignf(1e-20f, ray.d.x));
+    const float iy = 1.0f / (fabsf(ray.d.y) > 1e-20f ? ray.d.y : copysignf(1e-20f, ray.d.y));
+    const float iz = 1.0f / (fabsf(ray.d.z) > 1e-20f ? ray.d.z : copysignf(1e-20f, ray.d.z));
+    const unsigned long long ix2 = pair_of(ix), iy2 = pair_of(iy), iz2 = pair_of(iz);
+    const unsigned long long ox2 = pair_of(-ray.o.x * ix), oy2 = pair_of(-ray.o.y * iy), oz2 = pair_of(-ray.o.z * iz);
+    // the sphere class divides by |d|^2 once per walk instead of once per sphere test
+    float ia_ray = 0.0f;
+    if constexpr (SPH && !COUNT) ia_ray = 1.0f / len2(ray.d);
+    const ulonglong2* nodes = reinterpret_cast<const ulonglong2*>(S.nodes);
+    const uint32_t stride = blockDim.x * 4u;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(stack);
+    const uint32_t limit = base + (uint32_t)S.stack_depth * stride;
+    uint32_t sp = base + (uint32_t)tv.sp;      // address of the top entry
+    int node = act ? tv.node : kSentinel;      // inner node index, leaf (< 0) or kSentinel
+    int leaf = 0;                              // postponed leaf (< 0) or 0
+    for (;;) {
         for (;;) {
-            while ((unsigned)node < (unsigned)kSentinel) {
-                float4 n0 = __ldg(nodes + 4 * node + 0);
-                float4 n1 = __ldg(nodes + 4 * node + 1);
-                float4 n2 = __ldg(nodes + 4 * node + 2);
-                const int2 n3 = __ldg(reinterpret_cast<const int2*>(nodes + 4 * node + 3));
+            if ((unsigned)node < (unsigned)kSentinel) {
+                const ulonglong2 n0 = __ldg(nodes + 4 * node + 0), n1 = __ldg(nodes + 4 * node + 1),
+                                 n2 = __ldg(nodes + 4 * node + 2);
+                const int2 link = __ldg(reinterpret_cast<const int2*>(nodes + 4 * node + 3));
                 if constexpr (COUNT) tl->node++;
-                // slab tests of both children (aabb.rs:18-56)
-                float a0 = fmaf(n0.x, ix, ox), a1 = fmaf(n0.y, ix, ox);
-                float b0 = fmaf(n0.z, iy, oy), b1 = fmaf(n0.w, iy, oy);
-                float c0 = fmaf(n2.x, iz, oz), c1 = fmaf(n2.y, iz, oz);
-                float en0 = fmaxf(fmaxf(fminf(a0, a1), fminf(b0, b1)), fmaxf(fminf(c0, c1), tmin));
-                float ex0 = fminf(fminf(fmaxf(a0, a1), fmaxf(b0, b1)), fminf(fmaxf(c0, c1), hit.t));
-                float d0 = fmaf(n1.x, ix, ox), d1 = fmaf(n1.y, ix, ox);
-                float e0 = fmaf(n1.z, iy, oy), e1 = fmaf(n1.w, iy, oy);
-                float f0 = fmaf(n2.z, iz, oz), f1 = fmaf(n2.w, iz, oz);
-                float en1 = fmaxf(fmaxf(fminf(d0, d1), fminf(e0, e1)), fmaxf(fminf(f0, f1), tmin));
-                float ex1 = fminf(fminf(fmaxf(d0, d1), fmaxf(e0, e1)), fminf(fmaxf(f0, f1), hit.t));
+                // slab tests of both children (aabb.rs:18-56), lo and hi of an axis per pair
+                const float2 ax = fma_pair(n0.x, ix2, ox2), ay = fma_pair(n0.y, iy2, oy2), az = fma_pair(n2.x, iz2, oz2);
+                const float2 bx = fma_pair(n1.x, ix2, ox2), by = fma_pair(n1.y, iy2, oy2), bz = fma_pair(n2.y, iz2, oz2);
+                const float en0 = fmaxf(fmaxf(fminf(ax.x, ax.y), fminf(ay.x, ay.y)), fmaxf(fminf(az.x, az.y), tmin));
+                const float ex0 = fminf(fminf(fmaxf(ax.x, ax.y), fmaxf(ay.x, ay.y)), fminf(fmaxf(az.x, az.y), hit.t));
+                const float en1 = fmaxf(fmaxf(fminf(bx.x, bx.y), fminf(by.x, by.y)), fmaxf(fminf(bz.x, bz.y), tmin));
+                const float ex1 = fminf(fminf(fmaxf(bx.x, bx.y), fmaxf(by.x, by.y)), fminf(fmaxf(bz.x, bz.y), hit.t));
                 const bool h0 = en0 < ex0, h1 = en1 < ex1;
-                const int c0e = n3.x, c1e = n3.y;   // links: inner node or encoded leaf
-                if (!h0 && !h1) {
-                    node = sp > 0 ? stack[--sp * stride] : kSentinel;
-                } else {
-                    const bool first0 = h0 && (!h1 || en0 <= en1);
-                    node = first0 ? c0e : c1e;
-                    if (h0 && h1) {
-                        if (sp < S.stack_depth) {
-                            stack[sp++ * stride] = first0 ? c1e : c0e;
-                        } else {
-                            err |= LUM_KERR_STACK_OVERFLOW;
-                        }
+                const bool first0 = h0 && (!h1 || en0 <= en1);
+                const int far = first0 ? link.y : link.x;
+                node = first0 ? link.x : link.y;
+                const bool both = h0 && h1, none = !h0 && !h1, room = sp < limit;
+                if (both && !room) err |= LUM_KERR_STACK_OVERFLOW;
+                if (both && room) sp += stride;
+                store_if(both && room, sp, far);
+                load_if(none, sp, node);
+                if (none) sp -= stride;
+                const bool post = node < 0 && leaf == 0;
+                if (post) leaf = node;
+                load_if(post, sp, node);
+                if (post) sp -= stride;
+            }
+            // on while some lane that can walk has no leaf yet
+            if (!__any_sync(full, (unsigned)node < (unsigned)kSentinel && leaf == 0)) break;
+        }
+        int k = 0, last = -1;                  // primitives of the leaf to test
+        if (leaf < 0) {
+            k = (~leaf) >> 3;
+            last = k + ((~leaf) & 7);
+            leaf = 0;
+        }
+        while (__any_sync(full, k <= last)) {
+            if (k <= last) {
+                if (test_prim<COUNT, SPH, CLS>(S, k, ray, tmin, hit, tl, ia_ray)) {
+                    found = true;
+                    if (any) {                 // the shadow query is answered
+                        node = kSentinel;
+                        last = -1;
                     }
                 }
-                if (node < 0 && leaf == 0) {
-                    leaf = node;
-                    node = sp > 0 ? stack[--sp * stride] : kSentinel;
-                }
-                if (!__any_sync(__activemask(), leaf == 0)) break;
-            }
-            while (leaf < 0) {
-                const int first = (~leaf) >> 3, cnt = ((~leaf) & 7) + 1;
-                for (int k = 0; k < cnt; ++k) {
-                    if (test_prim<COUNT, SPH, CLS>(S, first + k, ray, tmin, hit, tl, ia_ray)) {
-                        found = true;
-                        if (any) {
-                            tv.node = kSentinel;
-                            return true;
-                        }
-                    }
-                }
-                leaf = 0;
-                if (node < 0) {
-                    leaf = node;
-                    node = sp > 0 ? stack[--sp * stride] : kSentinel;
-                }
-            }
-            if (node == kSentinel) break;
-            if constexpr (SUSPEND > 0) {
-                if (__popc(__activemask()) <= SUSPEND) {
-                    tv.node = node;
-                    tv.sp = sp;
-                    return false;
+                ++k;
+                if (k > last && node < 0) {    // the next node is a leaf too
+                    k = (~node) >> 3;
+                    last = k + ((~node) & 7);
+                    load_if(true, sp, node);
+                    sp -= stride;
                 }
             }
         }
-        tv.node = kSentinel;
+        if (__popc(__ballot_sync(full, node != kSentinel)) <= SUSPEND) break;
     }
-    for (int k = 0; k < S.n_planes; ++k) {                             // scene.rs:826-831
+    if (act) {
+        tv.node = node;
+        tv.sp = (int)(sp - base);
+    }
+    if (!act || node != kSentinel) return false;
+    for (int k = 0; k < S.n_planes && !(any && found); ++k) {              // scene.rs:826-831
         if constexpr (COUNT) tl->plane++;
         float t;
         if (hit_plane(S.planes[k], ray, tmin, hit.t, t)) {
             hit.t = t;
             hit.prim = -2 - k;
             found = true;
-            if (any) return true;
         }
     }
     return true;
@@ -493,7 +539,7 @@ __device__ __forceinline__ bool trace_resume(const SceneDev& S, const Ray& ray, 
 
 // LUM_SUSPEND_LANES, the SUSPEND of the persistent kernels' walks: lanes still walking the BVH
 // when at most that many of the warp are left keep their place and let the finished lanes shade
-// and start new rays first (trace_resume); 0 = every walk runs to its end before any lane
+// and start new rays first (walk_warp); 0 = every walk runs to its end before any lane
 // shades.  Measured on B200 against 0 (kernel time per frame, images
 // identical): 4 / 8 / 16 lanes gave the sphere field 101.7 -> 91.1 / 91.9 / 92.4 ms, the box room
 // 2.57 -> 2.40 / 2.29 / 2.23 ms, the quad scene 13.6 -> 11.5 / 11.4 / 11.8 ms and the dense mesh
@@ -504,13 +550,13 @@ __device__ __forceinline__ bool trace_resume(const SceneDev& S, const Ray& ray, 
 
 // Closest hit (any = false) keeps the nearest accepted t; any = true returns at the first
 // accepted hit (the shadow query, render.rs:1457-1460).  Unbounded planes follow the BVH
-// (scene.rs:826-831).
+// (scene.rs:826-831).  Called by the whole warp; act: the lane has a ray.
 template <bool COUNT = false, bool SPH = false>
 __device__ __forceinline__ bool trace(const SceneDev& S, const Ray& ray, float tmin, bool any, Hit& hit, int* stack,
-                                      uint32_t& err, TestTally* tl = nullptr) {
+                                      uint32_t& err, bool act, TestTally* tl = nullptr) {
     bool found = false;
     Trav tv{S.n_nodes > 0 ? 0 : kSentinel, 0};
-    trace_resume<COUNT, SPH, 0>(S, ray, tmin, any, hit, found, tv, stack, err, tl);
+    walk_warp<COUNT, SPH, 0>(S, ray, tmin, any, hit, found, tv, stack, err, act, tl);
     return found;
 }
 
@@ -1051,14 +1097,20 @@ __device__ __forceinline__ V envmap(const float* env, uint32_t env_w, uint32_t e
     return c * intensity;
 }
 
+// The unit direction and the gradients' blend are rounded explicitly (see add_light): an image must
+// not depend on which kernel's contraction of y * rsqrt + 1 or a * (1 - t) + b * t it got.
 template <bool EXT = true>
 __device__ __forceinline__ V background(const SceneDev& S, const RenderDev& R, const Ray& r) {  // render.rs:73-171
     if (R.background == 1) return mk(R.bg_color);
-    V ud = unit(r.d);
-    float t = 0.5f * (ud.y + 1.0f);
-    if (R.background == 2) return mk(R.bg_color) * (1.0f - t) + mk(R.bg_color2) * t;
+    const float rl = rsqrtf(len2(r.d));
+    const V ud = V{__fmul_rn(r.d.x, rl), __fmul_rn(r.d.y, rl), __fmul_rn(r.d.z, rl)};
+    const float t = 0.5f * __fadd_rn(ud.y, 1.0f), u = __fsub_rn(1.0f, t);
+    auto blend = [t, u](V a, V b) {
+        return V{fmaf(b.x, t, __fmul_rn(a.x, u)), fmaf(b.y, t, __fmul_rn(a.y, u)), fmaf(b.z, t, __fmul_rn(a.z, u))};
+    };
+    if (R.background == 2) return blend(mk(R.bg_color), mk(R.bg_color2));
     if (R.background == 3) {
-        V sky = mk(1.f, 1.f, 1.f) * (1.0f - t) + mk(R.bg_color2) * t;
+        V sky = blend(mk(1.f, 1.f, 1.f), mk(R.bg_color2));
         float sd = dot(ud, unit(mk(R.bg_dir)));
         if (sd > 0.9995f) return mk(R.bg_color) * R.bg_intensity;
         if (sd > 0.995f) {
@@ -1071,7 +1123,7 @@ __device__ __forceinline__ V background(const SceneDev& S, const RenderDev& R, c
         if (R.background == 4) return starfield(R.star_density, R.star_brightness, ud, t);
         if (R.background == 5) return envmap(S.env, S.env_w, S.env_h, R.bg_intensity, ud);
     }
-    return mk(1.f, 1.f, 1.f) * (1.0f - t) + mk(0.5f, 0.7f, 1.0f) * t;
+    return blend(mk(1.f, 1.f, 1.f), mk(0.5f, 0.7f, 1.0f));
 }
 
 // The pixel filter is written with explicitly rounded operations (no FMA contraction): the
@@ -1216,6 +1268,12 @@ __device__ __forceinline__ void shadow_done(Path& P, Pending& pend, const V* exi
     }
 }
 
+// L += B (.) e, fused explicitly: the compiler contracts the product and the sum or not depending on
+// the code around them, and every kernel must round a path's radiance alike.
+__device__ __forceinline__ void add_light(Path& P, V e) {
+    P.L = V{fmaf(P.beta.x, e.x, P.L.x), fmaf(P.beta.y, e.y, P.L.y), fmaf(P.beta.z, e.z, P.L.z)};
+}
+
 // Shading after the closest hit of segment j (ray_color, render.rs:1472-1537, iterative):
 // L += B_j e_j now, B_{j+1} = B_j att_j rrw_j, the NEE term B_j d_j once its shadow ray is
 // known to be unoccluded.  Returns the lane's next state.
@@ -1225,7 +1283,7 @@ template <int KIND = -1, bool EXT = true, bool NEE = true, bool SPH = false, int
 __device__ __forceinline__ int shade(const SceneDev& S, const RenderDev& R, uint32_t pixel, Path& P, bool found,
                                      const Hit& h, Pending& pend, V* exit_stash = nullptr) {
     if (!found) {
-        P.L = P.L + mul(P.beta, background<EXT>(S, R, P.ray));
+        add_light(P, background<EXT>(S, R, P.ray));
         return ST_DONE;
     }
     const uint32_t depth = R.max_depth - P.bounce;
@@ -1244,14 +1302,14 @@ __device__ __forceinline__ int shade(const SceneDev& S, const RenderDev& R, uint
     sc.org = sf.p;
     const MatDev& ms = EXT && KIND < 0 ? blend_leaf(S, m, R, pixel, P.stratum, P.bounce) : m;
     if (!scatter<KIND, EXT, SPH, philox_unroll<CLS>()>(ms, P.ray, sf, h.t, su, R, pixel, P.stratum, P.bounce, sc)) {
-        P.L = P.L + mul(P.beta, e);
+        add_light(P, e);
         return ST_DONE;
     }
     // A zero or non-finite scatter direction (in_unit_sphere at radius 0) would make the
     // next level NaN in the reference (its unit vectors divide by zero): end the path.
     const float dl2 = len2(sc.dir);
     if (!(dl2 > 0.0f) || !isfinite(dl2)) {
-        P.L = P.L + mul(P.beta, e);
+        add_light(P, e);
         return ST_DONE;
     }
     // the next segment (its origin and direction are dead past this point otherwise; a path
@@ -1261,13 +1319,13 @@ __device__ __forceinline__ int shade(const SceneDev& S, const RenderDev& R, uint
     float4 nu = draw4<philox_unroll<CLS>()>(R.key0, R.key1, pixel, P.stratum, P.bounce, CALL_NEE);
     float surv = fminf(fmaxf(fmaxf(fmaxf(sc.att.x, sc.att.y), sc.att.z), 0.05f), 1.0f);
     if (depth < 47 && nu.x > surv) {                                   // Russian roulette
-        P.L = P.L + mul(P.beta, e);
+        add_light(P, e);
         return ST_DONE;
     }
     float rrw = depth < 47 ? 1.0f / surv : 1.0f;
     V nb = mul(P.beta, sc.att) * rrw;
     if (has_nan(e) || has_nan(nb)) return ST_DONE;                     // render.rs:1526-1531
-    P.L = P.L + mul(P.beta, e);
+    add_light(P, e);
     bool use_nee = NEE && !m.specular && S.n_lights > 0;
     bool shadow = false;
     if (use_nee) {

@@ -197,14 +197,17 @@ __global__ void k_post_generate(Ctl* ctl) {
 
 __global__ void k_extend(Pool pl, Tables T, Ctl* ctl) {
     extern __shared__ int s_stack[];
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     const uint32_t cur = ctl->cur;
     const uint32_t n = ctl->ext_n[cur];
     const bool sorted = n >= T.sort_threshold;
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t err = 0, segs = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const uint32_t slot = pl.ext[cur][i];
+    // warps go on together: a lane past the end of the queue walks along without a ray
+    for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < n; w0 += stride) {
+        const uint32_t i = w0 + (threadIdx.x & 31u);
+        const bool live = i < n;
+        const uint32_t slot = pl.ext[cur][live ? i : w0];
         const float4 a = pl.o_t[slot], b = pl.d_jx[slot];
         const uint4 id = pl.ids[slot];
         const SceneDev S = T.scenes[id.x];
@@ -213,12 +216,11 @@ __global__ void k_extend(Pool pl, Tables T, Ctl* ctl) {
         h.t = CUDART_INF_F;
         h.prim = -1;
         h.b1 = h.b2 = 0.0f;
-        bool found = false;
-        if (bounce < T.renders[id.x].max_depth) {
-            Ray r{xyz(a), xyz(b), a.w};
-            found = trace(S, r, 0.001f, false, h, stack, err);
-            ++segs;
-        }
+        const bool act = live && bounce < T.renders[id.x].max_depth;
+        Ray r{xyz(a), xyz(b), a.w};
+        const bool found = trace(S, r, 0.001f, false, h, stack, err, act);
+        if (act) ++segs;
+        if (!live) continue;
         pl.hit[slot] = make_float4(h.t, __int_as_float(found ? h.prim : -1), h.b1, h.b2);
         int q = 0;
         if (found && sorted) {
@@ -286,12 +288,14 @@ __global__ void k_shade(Pool pl, Tables T, Ctl* ctl) {
 
 __global__ void k_shadow(Pool pl, Tables T, Ctl* ctl) {
     extern __shared__ int s_stack[];
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     const uint32_t n = ctl->shadow_n;
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t err = 0, cnt = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const uint32_t slot = pl.shadowq[i];
+    for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < n; w0 += stride) {
+        const uint32_t i = w0 + (threadIdx.x & 31u);
+        const bool live = i < n;
+        const uint32_t slot = pl.shadowq[live ? i : w0];
         const uint4 id = pl.ids[slot];
         const float4 sd = pl.sdir[slot], sc = pl.scon[slot];
         const int flags = (int)sc.w;
@@ -300,9 +304,10 @@ __global__ void k_shadow(Pool pl, Tables T, Ctl* ctl) {
         Hit h;
         h.t = sd.w;
         h.prim = -1;
-        ++cnt;
         const SceneDev S = T.scenes[id.x];
-        const bool occluded = trace(S, r, 0.001f, true, h, stack, err);
+        const bool occluded = trace(S, r, 0.001f, true, h, stack, err, live);
+        if (!live) continue;
+        ++cnt;
         if (!occluded) {
             float4 l = pl.L[slot];
             l.x += sc.x;
@@ -375,7 +380,7 @@ __global__ void __launch_bounds__(128, 5) k_render_multi(Tables T, const unsigne
     __shared__ unsigned long long s_acc[4][32][4];
     __shared__ uint32_t s_next[4];
     __shared__ V s_exit[4][32];                  // deferred Subsurface origins
-    int* stack = s_stack + threadIdx.x;
+    int* stack = lane_stack(s_stack);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned long long total = task_prefix[T.n];
     uint32_t err = 0, nseg = 0, nsh = 0;
@@ -752,7 +757,7 @@ lum_status create_batch(lum_scene* const* scenes, const lum_render_params* param
     if (!mega && (cfg.iters_per_graph < 1 || cfg.iters_per_graph > 64))
         return fail_out(lum::set_error(LUM_ERR_INVALID_ARGUMENT, "iters_per_graph out of range"));
     b->block = mega || lanes ? 128 : (int)cfg.block_threads;
-    b->stack_bytes = (size_t)lum::kStackDepth * b->block * sizeof(int);
+    b->stack_bytes = lum::stack_smem(lum::kStackDepth, b->block);
 
     // one allocation: pool SoA, queues, tables, accumulators, staging images
     size_t off = 0;
@@ -833,9 +838,9 @@ lum_status create_batch(lum_scene* const* scenes, const lum_render_params* param
     int occ_m = 0;
     for (auto fn : {k_render_multi<true>, k_render_multi<false>})
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)((size_t)lum::kStackDepth * 128 * sizeof(int)));
+                             (int)(lum::stack_smem(lum::kStackDepth, 128)));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_m, k_render_multi<true>, 128,
-                                                  (size_t)lum::kStackDepth * 128 * sizeof(int));
+                                                  lum::stack_smem(lum::kStackDepth, 128));
     b->grid_mega = sms * std::max(occ_m, 1);
 
     if (lanes) {
@@ -865,10 +870,10 @@ lum_status create_batch(lum_scene* const* scenes, const lum_render_params* param
         return fail_out(wf_cuda(e, "cudaStreamBeginCapture"));
     if (mega) {
         if (n <= kConstScenes)
-            k_render_multi<true><<<b->grid_mega, 128, (size_t)lum::kStackDepth * 128 * sizeof(int), b->stream>>>(
+            k_render_multi<true><<<b->grid_mega, 128, lum::stack_smem(lum::kStackDepth, 128), b->stream>>>(
                 b->T, b->d_tile_prefix, b->d_order, b->d_groups, b->ctl, b->d_next_task);
         else
-            k_render_multi<false><<<b->grid_mega, 128, (size_t)lum::kStackDepth * 128 * sizeof(int), b->stream>>>(
+            k_render_multi<false><<<b->grid_mega, 128, lum::stack_smem(lum::kStackDepth, 128), b->stream>>>(
                 b->T, b->d_tile_prefix, b->d_order, b->d_groups, b->ctl, b->d_next_task);
     } else {
         for (uint32_t g = 0; g < cfg.iters_per_graph; ++g) enqueue_iteration(b);

@@ -1,0 +1,46 @@
+"""GPU test of calls whose rays or pixels do not fill whole warps.
+
+The traversal walks a warp's rays together, lanes without a ray following along, so the results
+of a small or ragged call must equal those of the same rays and pixels inside a larger one, bit
+for bit: ray sets around the warp (32) and block (128) sizes, and crops smaller than an 8x4 tile.
+"""
+import numpy as np
+import pytest
+
+import luminara_b200 as L
+from luminara_b200 import workloads as W
+
+from .helpers import random_rays, to_gpu_rays
+
+pytestmark = pytest.mark.gpu
+
+SCENES = {"box_room": (lambda: W.box_room(64, 48, 4), (0, 0, 0), (555, 555, 555)),
+          "zoo": (lambda: W.material_zoo(64, 48, 4), (-6, 0, -4), (6, 8, 6)),
+          "mesh": (lambda: W.dense_mesh(64, 48, 4, level=3), (-2, -1, -2), (2, 2, 2))}
+
+
+@pytest.mark.parametrize("name", sorted(SCENES))
+def test_ragged_ray_sets_equal_the_whole_set(name):
+    build, lo, hi = SCENES[name]
+    sc = L.GpuScene(build()[0])
+    rays = to_gpu_rays(*random_rays(np.random.default_rng(3), 4097, lo, hi))
+    hits, occ = sc.intersect(rays), sc.occluded(rays)
+    assert 0 < occ.sum()
+    np.testing.assert_array_equal(occ != 0, hits["prim_id"] >= 0)
+    for n in (1, 31, 32, 33, 127, 128, 129, 1000):
+        assert sc.intersect(rays[:n]).tobytes() == hits[:n].tobytes(), n
+        np.testing.assert_array_equal(sc.occluded(rays[:n]), occ[:n])
+    sc.close()
+
+
+@pytest.mark.parametrize("name", sorted(SCENES))
+@pytest.mark.parametrize("crop", [(0, 0, 1, 1), (7, 3, 9, 5), (5, 6, 8, 4), (40, 30, 24, 18)])
+def test_ragged_crops_equal_the_frame(name, crop):
+    world, cfg = SCENES[name][0]()
+    sc = L.GpuScene(world)
+    frame, _ = sc.render(cfg)
+    cfg.crop = crop
+    part, _ = sc.render(cfg)
+    x, y, w, h = crop
+    np.testing.assert_array_equal(part, frame[y:y + h, x:x + w])
+    sc.close()
