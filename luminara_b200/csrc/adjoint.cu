@@ -648,9 +648,11 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                     tv.sp = 0;
                     found = false;
                 }
-                walking = !walk_warp<false, false, LUM_SUSPEND_LANES, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err,
-                                                                          act) && act;
-                if (walking || !act) {
+                const bool done = walk_warp<false, false, LUM_SUSPEND_LANES, CLS>(S, r, 0.001f, shadow, h, found, tv,
+                                                                                 stack, err, act);
+                walking = act && !done;
+                __syncwarp(kFullMask);   // the lanes shade together
+                if (!done) {
                     // no walk, or suspended: resumes in a later iteration
                 } else if (shadow) {
                     if (!found) {
@@ -689,6 +691,7 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                     state = stt == ST_SHADOW ? A_SHADOW : (stt == ST_CLOSEST ? A_CLOSEST : A_DONE);
                 }
             }
+            __syncwarp(kFullMask);
             if (state == A_DONE) {
                 PathHead ph;
                 ph.L = P.L;
@@ -702,6 +705,7 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                 heads[slot] = ph;
                 state = A_IDLE;
             }
+            __syncwarp(kFullMask);
         }
     }
     if (err) atomicOr(&wc->error_flags, err);

@@ -100,8 +100,8 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
             }
             state = ST_IDLE;
         }
+        __syncwarp(kAll);
     }
-    __syncwarp(kAll);
 }
 
 __global__ void k_stamp(WorkCounters* wc) { wc->t0_ns = globaltimer(); }

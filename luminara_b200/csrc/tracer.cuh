@@ -500,7 +500,7 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
             last = k + ((~leaf) & 7);
             leaf = 0;
         }
-        while (__any_sync(full, k <= last)) {
+        for (;;) {
             if (k <= last) {
                 if (test_prim<COUNT, SPH, CLS>(S, k, ray, tmin, hit, tl, ia_ray)) {
                     found = true;
@@ -517,6 +517,7 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
                     sp -= stride;
                 }
             }
+            if (!__any_sync(full, k <= last)) break;
         }
         if (__popc(__ballot_sync(full, node != kSentinel)) <= SUSPEND) break;
     }
