@@ -17,14 +17,14 @@
 
 namespace lum {
 
-// Primitive types (low 4 bits of meta)
+// Primitive types (low 4 bits of meta, and as an integer in c.w, which no type uses otherwise)
 enum PrimType : int32_t {
     PT_SPHERE = 0,    // a=(c, r)        b=(c1, moving?1:0)
-    PT_QUAD = 1,      // a=(Q, w.Q)      b=(u, |u x v|)    c=(v, 0)  d=(w, outward sign); w = (u x v)/|u x v|^2
-    PT_TRIANGLE = 2,  // a=(v0, 0)       b=(e1, 0)         c=(e2, 0) d=(n_geom, smooth-normal index or -1)
+    PT_QUAD = 1,      // a=(Q, w.Q)      b=(u, |u x v|)    c=(v, -)  d=(w, outward sign); w = (u x v)/|u x v|^2
+    PT_TRIANGLE = 2,  // a=(v0, 0)       b=(e1, 0)         c=(e2, -) d=(n_geom, smooth-normal index or -1)
     PT_DISK = 3,      // a=(c, r)        b=(n, 0)
-    PT_FOG_SPHERE = 4,// a=(c, r)        c=(neg_inv_density, 0, 0, 0)
-    PT_FOG_BOX = 5    // a=(min, 0)      b=(max, 0)        c=(neg_inv_density, 0, 0, 0)
+    PT_FOG_SPHERE = 4,// a=(c, r)        c=(neg_inv_density, 0, 0, -)
+    PT_FOG_BOX = 5    // a=(min, 0)      b=(max, 0)        c=(neg_inv_density, 0, 0, -)
 };
 
 constexpr int kStackDepth = 64;     // traversal stack entries per thread

@@ -921,6 +921,8 @@ lum_status lum_scene_create(const lum_scene_desc* desc, lum_scene** out) {
     for (size_t k = 0; k < np; ++k) {
         const PrimH& p = F.prims[bvh.order[k]];
         std::memcpy(&prims[16 * k], p.rec, sizeof p.rec);
+        const int32_t type = p.type;                 // record 2's w: the hit tests' type (device_scene.h)
+        std::memcpy(&prims[16 * k + 11], &type, sizeof type);
         meta[k] = (p.material << 4) | p.type;
         orig[k] = p.orig;
     }
