@@ -392,15 +392,57 @@ __device__ __forceinline__ int* lane_stack(int* smem) {
     return s;
 }
 
-// Shared-memory accesses (32-bit addresses) under a predicate rather than a branch: the lanes of
-// a visit that pop and those that push stay together.
-__device__ __forceinline__ void load_if(bool p, uint32_t addr, int& v) {
-    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\n@q ld.shared.b32 %0, [%1];\n}"
-                 : "+r"(v) : "r"(addr), "r"((int)p) : "memory");
+// The end of a node visit, given both children's slab intervals: the nearer child hit becomes the
+// node, the other one is pushed (or, past `limit`, dropped with the overflow flag); with no child
+// hit the node is popped; a node that is a leaf becomes the postponed leaf if there is none, and
+// another is popped.  sp: 32-bit shared address of the top entry.  One block of predicated
+// instructions: no branches, so the lanes that pop and those that push stay together, and no
+// predicate is turned into an integer and back (the integer pipe is the busiest, 63-67%): against
+// predicated accesses taking 0/1 operands 20.8 -> 20.3 ms on the sphere field (64 spp), 1% on quads
+// and the box room.
+__device__ __forceinline__ void visit_children(float en0, float ex0, float en1, float ex1, int link0, int link1,
+                                               int& node, int& leaf, uint32_t& sp, uint32_t limit, uint32_t stride,
+                                               uint32_t& err) {
+    asm volatile(
+        "{\n"
+        ".reg .pred h0, h1, c1, both, none, room, push, over, post;\n"
+        ".reg .b32 n, f;\n"
+        "setp.lt.f32 h0, %4, %5;\n"
+        "setp.lt.f32 h1, %6, %7;\n"
+        "setp.lt.f32 c1, %6, %4;\n"          // child 1 first: h1 && (!h0 || en1 < en0)
+        "not.pred none, h0;\n"
+        "or.pred c1, c1, none;\n"
+        "and.pred c1, c1, h1;\n"
+        "and.pred both, h0, h1;\n"
+        "or.pred none, h0, h1;\n"
+        "not.pred none, none;\n"
+        "selp.b32 n, %9, %8, c1;\n"
+        "selp.b32 f, %8, %9, c1;\n"
+        "setp.lt.u32 room, %2, %10;\n"
+        "and.pred push, both, room;\n"
+        "not.pred room, room;\n"
+        "and.pred over, both, room;\n"
+        "@over or.b32 %3, %3, %12;\n"
+        "@push add.u32 %2, %2, %11;\n"
+        "@push st.shared.b32 [%2], f;\n"
+        "@none ld.shared.b32 n, [%2];\n"
+        "@none sub.u32 %2, %2, %11;\n"
+        "setp.lt.s32 post, n, 0;\n"
+        "setp.eq.and.s32 post, %1, 0, post;\n"
+        "@post mov.b32 %1, n;\n"
+        "@post ld.shared.b32 n, [%2];\n"
+        "@post sub.u32 %2, %2, %11;\n"
+        "mov.b32 %0, n;\n"
+        "}"
+        : "=r"(node), "+r"(leaf), "+r"(sp), "+r"(err)
+        : "f"(en0), "f"(ex0), "f"(en1), "f"(ex1), "r"(link0), "r"(link1), "r"(limit), "r"(stride),
+          "n"((int)LUM_KERR_STACK_OVERFLOW)
+        : "memory");
 }
-__device__ __forceinline__ void store_if(bool p, uint32_t addr, int v) {
-    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\n@q st.shared.b32 [%0], %1;\n}"
-                 :: "r"(addr), "r"(v), "r"((int)p) : "memory");
+__device__ __forceinline__ int load_shared(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
 }
 
 // Two f32 fused multiply-adds in one instruction (each rounded as fmaf rounds).
@@ -415,6 +457,7 @@ __device__ __forceinline__ float2 fma_pair(unsigned long long a, unsigned long l
         : "=f"(r.x), "=f"(r.y) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+
 
 // Place of a suspended BVH walk (walk_warp): the next node to visit (an inner node index, or
 // kSentinel when the walk is over) and the stack's depth in bytes; the stack entries stay in
@@ -434,7 +477,7 @@ struct Trav {
 //
 // What bounds it is instruction issue and how many lanes each instruction serves.  So both loops
 // are the warp's: their conditions are full-warp votes, which also bring the lanes together
-// after every visit and every primitive test; the stack is moved by predicated accesses; a leaf's
+// after every visit and every primitive test; a visit ends without branches (visit_children); a leaf's
 // primitives and a second pending leaf follow each other in one loop, so a lane with a short
 // leaf takes its next one meanwhile; and the slab tests use the packed f32 FMA.  The earlier form
 // (each lane's own loops, which the compiler let diverge: 11.4 lanes per instruction on the box
@@ -444,7 +487,7 @@ struct Trav {
 // Leaving the node loop once at most 3 lanes lack a leaf gained 1-2% on the sphere field and the
 // mesh and lost 7-9% on the room and the materials' scene; leaving it only when no lane can
 // walk on (no vote on leaves) lost 4-13%; leaving the leaf loop with 2, 6 or 12 lanes' leaves
-// unfinished lost 2-10%; branches instead of the predicated accesses lost up to 3%.
+// unfinished lost 2-10%; branches instead of predicated stack accesses lost up to 3%.
 template <bool COUNT = false, bool SPH = false, int SUSPEND = 0, int CLS = CLS_ALL>
 __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, float tmin, bool any, Hit& hit,
                                           bool& found, Trav& tv, int* stack, uint32_t& err, bool act,
@@ -482,20 +525,7 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
                 const float ex0 = fminf(fminf(fmaxf(ax.x, ax.y), fmaxf(ay.x, ay.y)), fminf(fmaxf(az.x, az.y), hit.t));
                 const float en1 = fmaxf(fmaxf(fminf(bx.x, bx.y), fminf(by.x, by.y)), fmaxf(fminf(bz.x, bz.y), tmin));
                 const float ex1 = fminf(fminf(fmaxf(bx.x, bx.y), fmaxf(by.x, by.y)), fminf(fmaxf(bz.x, bz.y), hit.t));
-                const bool h0 = en0 < ex0, h1 = en1 < ex1;
-                const bool first0 = h0 && (!h1 || en0 <= en1);
-                const int far = first0 ? link.y : link.x;
-                node = first0 ? link.x : link.y;
-                const bool both = h0 && h1, none = !h0 && !h1, room = sp < limit;
-                if (both && !room) err |= LUM_KERR_STACK_OVERFLOW;
-                if (both && room) sp += stride;
-                store_if(both && room, sp, far);
-                load_if(none, sp, node);
-                if (none) sp -= stride;
-                const bool post = node < 0 && leaf == 0;
-                if (post) leaf = node;
-                load_if(post, sp, node);
-                if (post) sp -= stride;
+                visit_children(en0, ex0, en1, ex1, link.x, link.y, node, leaf, sp, limit, stride, err);
             }
             // on while some lane that can walk has no leaf yet
             if (!__any_sync(full, (unsigned)node < (unsigned)kSentinel && leaf == 0)) break;
@@ -519,7 +549,7 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
                 if (k > last && node < 0) {    // the next node is a leaf too
                     k = (~node) >> 3;
                     last = k + ((~node) & 7);
-                    load_if(true, sp, node);
+                    node = load_shared(sp);
                     sp -= stride;
                 }
             }
