@@ -173,7 +173,9 @@ struct RenderDev {
     uint32_t tiles_x, n_tasks;
     float star_density, star_brightness;   // STARFIELD background
     uint32_t ext;            // the scene or background uses the other materials / backgrounds
-    uint32_t pad_ext;
+    uint32_t root_magic;     // ceil(2^32 / sqrt_spp): stratum / sqrt_spp by a high multiply (0: divide)
+    float inv_root;          // 1 / sqrt_spp
+    float inv_w1, inv_h1;    // 1 / (full_w - 1), 1 / (full_h - 1) (0 for an extent of 1)
 };
 
 }  // namespace lum

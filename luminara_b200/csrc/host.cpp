@@ -754,6 +754,11 @@ lum_status make_render_dev(const lum_scene* s, const lum_render_params& p, lum::
     if ((uint64_t)R.full_w * R.full_h > 0xFFFFFFFFull) return fail(LUM_ERR_TOO_LARGE, "image has more than 2^32 pixels");
     R.sqrt_spp = (uint32_t)std::ceil(std::sqrt((double)p.samples_per_pixel));   // render.rs:1589
     uint32_t total = R.sqrt_spp * R.sqrt_spp;
+    // st * ceil(2^32 / root) >> 32 is st / root while st * root < 2^32: st < root^2, so root <= 1625
+    R.root_magic = R.sqrt_spp >= 2 && R.sqrt_spp <= 1625 ? (uint32_t)(((1ull << 32) + R.sqrt_spp - 1) / R.sqrt_spp) : 0;
+    R.inv_root = 1.0f / (float)R.sqrt_spp;
+    R.inv_w1 = R.full_w > 1 ? 1.0f / (float)(R.full_w - 1) : 0.0f;
+    R.inv_h1 = R.full_h > 1 ? 1.0f / (float)(R.full_h - 1) : 0.0f;
     R.s_begin = std::min(p.sample_begin, total);
     R.s_end = p.sample_count ? std::min(total, R.s_begin + p.sample_count) : total;
     R.max_depth = p.max_depth;

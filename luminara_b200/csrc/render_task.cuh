@@ -121,9 +121,19 @@ __device__ __forceinline__ void tile_task(const SceneDev& S, const RenderDev& R,
         if (state == ST_IDLE) {
             const uint32_t idx = atomicAdd(next, 1u);
             if (idx < n_items) {
-                cur = idx % nv;
-                const uint32_t st = s_lo + idx / nv;
-                const uint32_t gi = x0 + cur % tw + R.crop_x, gj = y0 + cur / tw + R.crop_y;
+                uint32_t st, px, py;
+                if (nv == 32u) {          // a whole 8x4 tile
+                    cur = idx & 31u;
+                    st = s_lo + (idx >> 5);
+                    px = cur & 7u;
+                    py = cur >> 3;
+                } else {
+                    cur = idx % nv;
+                    st = s_lo + idx / nv;
+                    px = cur % tw;
+                    py = cur / tw;
+                }
+                const uint32_t gi = x0 + px + R.crop_x, gj = y0 + py + R.crop_y;
                 pixel = gj * R.full_w + gi;
                 start_path<philox_unroll<CLS>()>(S, R, gi, gj, pixel, st, P);
                 state = R.max_depth > 0 ? ST_CLOSEST : ST_DONE;
@@ -137,11 +147,14 @@ __device__ __forceinline__ void tile_task(const SceneDev& S, const RenderDev& R,
             add_fixed(&acc[cur][0], v.x);
             add_fixed(&acc[cur][1], v.y);
             add_fixed(&acc[cur][2], v.z);
-            add_fixed(&acc[cur][3], v.w);
+            if (R.pixel_filter != LUM_FILTER_BOX) add_fixed(&acc[cur][3], v.w);
             state = ST_IDLE;
         }
         __syncwarp(full);
     }
+    // the box filter weighs every path 1: a pixel's weight is its count of strata
+    if (R.pixel_filter == LUM_FILTER_BOX && lane < (int)nv) acc[lane][3] = (uint64_t)(s_hi > s_lo ? s_hi - s_lo : 0u) << 32;
+    __syncwarp(full);
 }
 
 }  // namespace lum

@@ -44,3 +44,19 @@ def test_ragged_crops_equal_the_frame(name, crop):
     x, y, w, h = crop
     np.testing.assert_array_equal(part, frame[y:y + h, x:x + w])
     sc.close()
+
+
+def test_small_frames_and_strata_match_the_keyed_oracle():
+    """Widths, heights and stratum counts around the tile (8x4) and the divisions of a path start."""
+    import oracle as O
+    close = total = 0
+    for w, h in [(2, 2), (3, 5), (8, 4), (17, 9), (33, 2)]:
+        for spp in (1, 3, 16, 30):
+            world, cfg = W.box_room(w, h, spp, seed=100 * w + spp)
+            sc = L.GpuScene(world)
+            img, _ = sc.render(cfg)
+            sc.close()
+            ref = O.OracleScene(world).render(cfg, mode=O.MODE_KEYED)[0]
+            near = (np.abs(img - ref) <= 2e-3 * (1 + np.abs(ref))).all(-1)   # the keyed renders' rule
+            close, total = close + int(near.sum()), total + near.size
+    assert close >= 0.97 * total, (close, total)
