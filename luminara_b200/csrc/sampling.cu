@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -50,7 +51,7 @@ __device__ __forceinline__ V clamp_sample(V L) {
 // filter-weighted value to acc[tile pixel] in fixed point (tile_task's sums; the call zeroes
 // acc); without, its clamped sample goes to smp[stratum - st_lo][tile pixel].  One copy of
 // the traversal and shading code serves every kind of tile.
-template <bool EXT, bool NEE, bool SPH>
+template <bool EXT, bool NEE, bool SPH, int CLS>
 __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& R, uint32_t x0, uint32_t y0, uint32_t tw,
                             const uint32_t* slot_px, uint32_t n_slots, uint32_t st_lo, uint32_t n_st, bool centre,
                             unsigned long long (*acc)[4], float (*smp)[32][3], uint32_t* next, V* exit_stash,
@@ -60,6 +61,8 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
     if (lane == 0) *next = 0u;
     __syncwarp(kAll);
     const uint32_t n_items = n_slots * n_st;
+    // idx / n_slots by a high multiply (exact for idx * n_slots < 2^32); 0: one slot
+    const uint32_t magic = n_slots > 1 ? 0xFFFFFFFFu / n_slots + 1u : 0u;
     int state = ST_IDLE;
     uint32_t px = 0, k = 0, pixel = 0;
     Path P;
@@ -71,20 +74,21 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
         if (state == ST_IDLE) {
             const uint32_t idx = atomicAdd(next, 1u);
             if (idx < n_items) {
-                px = slot_px[idx % n_slots];
-                k = idx / n_slots;
-                const uint32_t gi = x0 + px % tw + R.crop_x, gj = y0 + px / tw + R.crop_y;
+                k = magic ? __umulhi(idx, magic) : idx;
+                px = slot_px[idx - k * n_slots];
+                const uint32_t row = tw == 8u ? px >> 3 : px / tw;
+                const uint32_t gi = x0 + px - row * tw + R.crop_x, gj = y0 + row + R.crop_y;
                 pixel = gj * R.full_w + gi;
                 if (centre)
                     start_path_centre(S, R, gi, gj, pixel, P);
                 else
-                    start_path(S, R, gi, gj, pixel, st_lo + k, P);
+                    start_path<philox_unroll<CLS>()>(S, R, gi, gj, pixel, st_lo + k, P);
                 state = R.max_depth > 0 ? ST_CLOSEST : ST_DONE;
             }
         }
         if (!__any_sync(kAll, state != ST_IDLE)) break;
-        path_step<false, EXT, NEE, SPH, LUM_SUSPEND_LANES, CLS_ALL>(S, R, pixel, state, P, pend, h, tv, found, walking,
-                                                                   exit_stash + lane, stack, err, nseg, nsh, nullptr);
+        path_step<false, EXT, NEE, SPH, LUM_SUSPEND_LANES, CLS>(S, R, pixel, state, P, pend, h, tv, found, walking,
+                                                               exit_stash + lane, stack, err, nseg, nsh, nullptr);
         if (state == ST_DONE) {
             if (acc) {
                 const float4 v = path_sample(R, P.L, P.jx, P.jy);
@@ -104,17 +108,30 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
     }
 }
 
+// a / n with r = 1 / n, correctly rounded (tracer.cuh's div_by in f64).
+__device__ __forceinline__ double div_by(double a, double n, double r) {
+    const double q = a * r;
+    return fma(fma(-q, n, a), r, q);
+}
+
 __global__ void k_stamp(WorkCounters* wc) { wc->t0_ns = globaltimer(); }
 
-template <bool ADAPTIVE, bool EXT, bool NEE, bool SPH>
-__global__ void __launch_bounds__(kSampThreads, ADAPTIVE ? 4 : 5) k_render_sampled(SceneDev S, RenderDev R, SamplingDev A,
+// Built per scene class like the megakernel.  The adaptive variant is bound by the warps it keeps
+// resident (118 registers, 16% of the warps active, with Welford's state in registers across the
+// traced rounds): the state sits in shared memory (5 KiB a block beside 24 KiB of samples), and
+// one reciprocal serves a sample's four divisions.  4 / 5 / 6 / 7 blocks/SM: sphere field 1080p 100
+// spp 28.8 / 26.4 / 27.0 / 27.6 ms (29.7 before), box room 512x512 3.80 / 3.77 / 3.84 / 4.01 (5.47),
+// mesh 960x540 11.8 / 11.4 / 11.9 / 12.3 (12.6).
+template <bool ADAPTIVE, bool EXT, bool NEE, bool SPH, int CLS>
+__global__ void __launch_bounds__(kSampThreads, ADAPTIVE ? 5 : 7) k_render_sampled(SceneDev S, RenderDev R, SamplingDev A,
                                                                     float* __restrict__ out, WorkCounters* wc) {
     extern __shared__ int s_stack[];
-    __shared__ unsigned long long s_acc[kSampWarps][32][4];
+    __shared__ unsigned long long s_acc[ADAPTIVE ? 1 : kSampWarps][32][4];
+    __shared__ double s_welford[ADAPTIVE ? kSampWarps : 1][5][32];
     __shared__ float s_smp[kSampWarps][ADAPTIVE ? kRoundStrata : 1][32][3];
     __shared__ uint32_t s_slot[kSampWarps][32];
     __shared__ uint32_t s_next[kSampWarps];
-    __shared__ V s_exit[kSampWarps][32];            // deferred Subsurface origins
+    __shared__ V s_exit[EXT ? kSampWarps : 1][32];  // deferred Subsurface origins
     int* stack = lane_stack(s_stack);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t err = 0, nseg = 0, nsh = 0;
@@ -136,7 +153,9 @@ __global__ void __launch_bounds__(kSampThreads, ADAPTIVE ? 4 : 5) k_render_sampl
         // expired tile is one round of centre samples, a tile without adaptive sampling one
         // round of all its strata into the fixed-point sums, an adaptive tile rounds of
         // kRoundStrata strata over its active pixels.
-        double mean_lum = 0.0, m2_lum = 0.0, mean[3] = {0.0, 0.0, 0.0};   // Welford (render.rs:1628-1667)
+        double (*wf)[32] = s_welford[ADAPTIVE ? wid : 0];   // Welford state (render.rs:1628-1667)
+        if constexpr (ADAPTIVE)
+            for (int q = 0; q < 5; ++q) wf[q][lane] = 0.0;
         uint32_t n = 0;
         bool active = o != nullptr;
         const bool fixed_sums = !ADAPTIVE && !expired;
@@ -146,27 +165,30 @@ __global__ void __launch_bounds__(kSampThreads, ADAPTIVE ? 4 : 5) k_render_sampl
             if (active) s_slot[wid][__popc(act & ((1u << lane) - 1u))] = lane;
             const uint32_t st_lo = expired ? 0u : ADAPTIVE ? lo : R.s_begin;
             const uint32_t n_st = expired ? 1u : ADAPTIVE ? min(kRoundStrata, total - lo) : R.s_end - R.s_begin;
-            sample_pool<EXT, NEE, SPH>(S, R, x0, y0, tw, s_slot[wid], __popc(act), st_lo, n_st, expired != 0,
-                        fixed_sums ? s_acc[wid] : nullptr, s_smp[wid], &s_next[wid], s_exit[wid], stack, err, nseg,
-                        nsh);
+            sample_pool<EXT, NEE, SPH, CLS>(S, R, x0, y0, tw, s_slot[wid], __popc(act), st_lo, n_st, expired != 0,
+                                            fixed_sums ? s_acc[ADAPTIVE ? 0 : wid] : nullptr, s_smp[wid], &s_next[wid],
+                                            s_exit[EXT ? wid : 0], stack, err, nseg, nsh);
             if (active) {
                 if (expired) {
                     for (int c = 0; c < 3; ++c) o[c] = s_smp[wid][0][lane][c] * R.exposure;
                     kept += 1;
                     active = false;
                 } else if (!ADAPTIVE) {
-                    fixed_pixel(s_acc[wid][lane], R.exposure, o);
+                    fixed_pixel(s_acc[ADAPTIVE ? 0 : wid][lane], R.exposure, o);
                     kept += n_st;
                     active = false;
                 } else {
+                    double mean_lum = wf[0][lane], m2_lum = wf[1][lane];
+                    double mean[3] = {wf[2][lane], wf[3][lane], wf[4][lane]};
                     for (uint32_t k = 0; k < n_st; ++k) {
                         const float* c = s_smp[wid][k][lane];
                         ++n;
+                        const double dn = (double)n, rn = 1.0 / dn;
                         const double lum = 0.2126 * (double)c[0] + 0.7152 * (double)c[1] + 0.0722 * (double)c[2];
                         const double d1 = lum - mean_lum;
-                        mean_lum += d1 / (double)n;
+                        mean_lum += div_by(d1, dn, rn);
                         m2_lum += d1 * (lum - mean_lum);
-                        for (int q = 0; q < 3; ++q) mean[q] += ((double)c[q] - mean[q]) / (double)n;
+                        for (int q = 0; q < 3; ++q) mean[q] += div_by((double)c[q] - mean[q], dn, rn);
                         if (n >= A.min_samples && n > 1 && sqrt(m2_lum / (double)(n - 1) / (double)n) < A.threshold) {
                             active = false;
                             break;
@@ -177,6 +199,9 @@ __global__ void __launch_bounds__(kSampThreads, ADAPTIVE ? 4 : 5) k_render_sampl
                         for (int q = 0; q < 3; ++q) o[q] = (float)mean[q] * R.exposure;
                         kept += n;
                     }
+                    wf[0][lane] = mean_lum;
+                    wf[1][lane] = m2_lum;
+                    for (int q = 0; q < 3; ++q) wf[2 + q][lane] = mean[q];
                 }
             }
             __syncwarp(kAll);   // the round's results are read before the next round writes
@@ -209,7 +234,7 @@ int num_sms() {
     return n;
 }
 
-template <bool ADAPTIVE, bool EXT, bool NEE, bool SPH>
+template <bool ADAPTIVE, bool EXT, bool NEE, bool SPH, int CLS>
 cudaError_t launch_t(const SceneDev& S, const RenderDev& R, const SamplingDev& A, float* out, WorkCounters* wc,
                      cudaStream_t stream) {
     // the traversal stack sized to the scene's BVH; resident blocks per stack size (cached)
@@ -221,14 +246,14 @@ cudaError_t launch_t(const SceneDev& S, const RenderDev& R, const SamplingDev& A
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!attr) {
-            cudaFuncSetAttribute(k_render_sampled<ADAPTIVE, EXT, NEE, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(k_render_sampled<ADAPTIVE, EXT, NEE, SPH, CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)stack_smem(kStackDepth, kSampThreads));
             attr = true;
         }
         for (const auto& e : occ_of)
             if (e.first == stack) occ = e.second;
         if (occ <= 0) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_render_sampled<ADAPTIVE, EXT, NEE, SPH>, kSampThreads,
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_render_sampled<ADAPTIVE, EXT, NEE, SPH, CLS>, kSampThreads,
                                                           stack);
             if (occ <= 0) occ = 1;
             occ_of.push_back({stack, occ});
@@ -238,7 +263,7 @@ cudaError_t launch_t(const SceneDev& S, const RenderDev& R, const SamplingDev& A
     int grid = num_sms() * occ;
     const int needed = (int)std::min<uint64_t>(((uint64_t)R.n_tasks + kSampWarps - 1) / kSampWarps, 1u << 30);
     grid = std::max(1, std::min(grid, needed));
-    k_render_sampled<ADAPTIVE, EXT, NEE, SPH><<<grid, kSampThreads, stack, stream>>>(S, R, A, out, wc);
+    k_render_sampled<ADAPTIVE, EXT, NEE, SPH, CLS><<<grid, kSampThreads, stack, stream>>>(S, R, A, out, wc);
     return cudaGetLastError();
 }
 
@@ -248,26 +273,23 @@ cudaError_t launch_render_sampled(const SceneDev& S, const RenderDev& R, const S
                                   WorkCounters* wc, cudaStream_t stream) {
     // scenes without the other materials and backgrounds, without lights, or made of spheres
     // with the basic materials run kernels built without the code they cannot reach
-    const bool nee = S.n_lights > 0;
-    if (R.ext) {
+    const bool nee = S.n_lights > 0, ad = A.adaptive != 0;
+    auto go = [&](auto ext, auto sph, auto cls) {
+        constexpr bool E = decltype(ext)::value, P = decltype(sph)::value;
+        constexpr int C = decltype(cls)::value;
         if (nee)
-            return A.adaptive ? launch_t<true, true, true, false>(S, R, A, out, wc, stream)
-                              : launch_t<false, true, true, false>(S, R, A, out, wc, stream);
-        return A.adaptive ? launch_t<true, true, false, false>(S, R, A, out, wc, stream)
-                          : launch_t<false, true, false, false>(S, R, A, out, wc, stream);
-    }
-    if (S.spheres_basic) {
-        if (nee)
-            return A.adaptive ? launch_t<true, false, true, true>(S, R, A, out, wc, stream)
-                              : launch_t<false, false, true, true>(S, R, A, out, wc, stream);
-        return A.adaptive ? launch_t<true, false, false, true>(S, R, A, out, wc, stream)
-                          : launch_t<false, false, false, true>(S, R, A, out, wc, stream);
-    }
-    if (nee)
-        return A.adaptive ? launch_t<true, false, true, false>(S, R, A, out, wc, stream)
-                          : launch_t<false, false, true, false>(S, R, A, out, wc, stream);
-    return A.adaptive ? launch_t<true, false, false, false>(S, R, A, out, wc, stream)
-                      : launch_t<false, false, false, false>(S, R, A, out, wc, stream);
+            return ad ? launch_t<true, E, true, P, C>(S, R, A, out, wc, stream)
+                      : launch_t<false, E, true, P, C>(S, R, A, out, wc, stream);
+        return ad ? launch_t<true, E, false, P, C>(S, R, A, out, wc, stream)
+                  : launch_t<false, E, false, P, C>(S, R, A, out, wc, stream);
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    if (R.ext) return go(Yes(), No(), std::integral_constant<int, CLS_ALL>());
+    if (S.spheres_basic) return go(No(), Yes(), std::integral_constant<int, CLS_ALL>());
+    if (S.cls == CLS_QUAD) return go(No(), No(), std::integral_constant<int, CLS_QUAD>());
+    if (S.cls == CLS_MESH) return go(No(), No(), std::integral_constant<int, CLS_MESH>());
+    return go(No(), No(), std::integral_constant<int, CLS_ALL>());
 }
 
 }  // namespace lum

@@ -60,3 +60,20 @@ def test_small_frames_and_strata_match_the_keyed_oracle():
             near = (np.abs(img - ref) <= 2e-3 * (1 + np.abs(ref))).all(-1)   # the keyed renders' rule
             close, total = close + int(near.sum()), total + near.size
     assert close >= 0.97 * total, (close, total)
+
+
+@pytest.mark.parametrize("name", sorted(SCENES))
+@pytest.mark.parametrize("size", [(1, 1), (37, 21), (64, 48)])
+def test_adaptive_without_stops_equals_the_plain_render(name, size):
+    """Threshold 0 never stops a pixel: the mean of all strata, which the plain render's box filter
+    gives too (f64 running mean against fixed-point sums: 2e-6, as for the other adaptive tests).
+    The mesh goes without its fog, whose free-flight distance hashes a ray's last bits."""
+    world, cfg = W.dense_mesh(64, 48, 4, level=3, fog=False) if name == "mesh" else SCENES[name][0]()
+    cfg.width, cfg.height, cfg.samples_per_pixel = size[0], size[1], 20     # 25 strata: rounds of 16 and 9
+    sc = L.GpuScene(world)
+    plain, _ = sc.render(cfg)
+    cfg.adaptive, cfg.adaptive_threshold = True, 0.0
+    img, st = sc.render(cfg)
+    sc.close()
+    assert st.paths == 25 * size[0] * size[1]
+    np.testing.assert_allclose(img, plain, rtol=2e-6, atol=2e-6)
