@@ -118,3 +118,22 @@ def test_power_of_two_exposure_integer_keys(exposure):
     want = OT.tonemap(img, {"exposure": exposure})
     compare(got, want)
     np.testing.assert_array_equal(got.reshape(-1, 4)[:4, :3].reshape(-1), want.reshape(-1, 4)[:4, :3].reshape(-1))
+
+
+@pytest.mark.parametrize("curve", [OT.ACES, OT.REINHARD, OT.FILMIC, OT.NONE])
+@pytest.mark.parametrize("exposure", [1.0, 2.0 ** -20, 2.0 ** 19, 2.0 ** 20, 1.7, 0.0])
+def test_common_chain_over_tiles_and_rare_values(curve, exposure):
+    """Pixel counts around the 4-pixel groups and 128-pixel tiles, with zeros, negatives, denormals,
+    huge values, infinities and NaN among them, at exposures on both sides of each key form."""
+    import torch
+    rare = np.array([0.0, -0.0, -1.0, 1e-45, 1e-38, 3.4e38, np.inf, -np.inf, np.nan, 1e29, 2.0 ** 97], np.float32)
+    for n in (1, 3, 4, 127, 128, 131, 516, 5003):
+        img = hdr_image(1, n, n) / np.float32(exposure if exposure > 0 else 1.0)
+        flat = img.reshape(-1)
+        flat[:: 7][: len(rare)] = rare[: len(flat[::7])]
+        d_hdr, d_out = torch.from_numpy(img).cuda(), torch.zeros((1, n, 4), dtype=torch.uint8, device="cuda")
+        chain = {"tone_map": curve, "exposure": exposure}
+        L.tonemap_device(d_hdr.data_ptr(), n, 1, tm_config(chain), 0, d_out.data_ptr())
+        torch.cuda.synchronize()
+        with np.errstate(all="ignore"):
+            compare(d_out.cpu().numpy(), OT.tonemap(img, chain))
