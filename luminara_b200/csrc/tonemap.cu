@@ -15,8 +15,10 @@
 //   k_tonemap  4 pixels per thread: three 16-byte loads of 12 floats, one 16-byte store of
 //              4 RGBA pixels (a scalar tail with byte stores for pixel counts not divisible
 //              by 4, or for buffers that are not 16-byte aligned).  With auto-exposure each block first
-//              sums the 256 partials in the same fixed order.  Chains with optional steps, and
-//              tone curves whose table does not fit, take the f32 path with its f64 fallback.
+//              sums the 256 partials in the same fixed order.  Dithered chains, unaligned buffers and
+//              tone curves whose table does not fit take the f32 path with its f64 fallback.
+//   k_tonemap_graded  chains with the other optional steps on 16-byte aligned buffers: colour steps
+//              in f64, byte tables for the rest.
 //   k_tonemap_flat  the common chain (no optional step) on 16-byte aligned buffers: each channel's
 //              byte from a table of the chain's 255 byte thresholds (one entry lookup per
 //              channel, see ByteTable).
@@ -39,6 +41,7 @@ namespace tone {
 
 constexpr int kLogBlocks = 256;
 constexpr int kLogThreads = 256;
+constexpr int kLogAhead = 8;          // steps of k_loglum whose loads are in flight together
 constexpr int kThreads = 256;
 static_assert(kLogBlocks * sizeof(double) <= LUM_TONEMAP_SCRATCH_BYTES, "scratch too small");
 
@@ -49,6 +52,8 @@ struct Chain {
     bool wb, hue, sat, grade, bright, contrast, sepia, tint, balance;
     bool extra;                   // any step beyond exposure, tone curve and gamma
     float inv_gamma;              // 1/gamma, or 0 for the sRGB transfer function
+    double wb_r, wb_g, wb_b;      // white-balance factors
+    double hue_d, hue_m, hue_p;   // hue rotation matrix (a circulant)
 };
 
 // Rust's `as u8` from f64: truncation, saturating, NaN -> 0.
@@ -138,29 +143,23 @@ __device__ __forceinline__ uint32_t tone_gamma(int kind, double x, double gamma,
     return q < 0.0 ? 0u : sat_u8(q);
 }
 
-// One pixel of the full chain (src/render.rs:3100-3260); pixel p = j * w + i of the output.
-__device__ __noinline__ uint32_t pixel_full(const Chain& C, double r, double g, double b, uint32_t p, uint32_t w,
-                                            uint32_t h, double exposure) {
+// a / b for a finite a and b = 1, 2, ... with r = 1 / b: the quotient corrected by its exact remainder
+// is the correctly rounded one (Markstein, IBM J. Res. Dev. 1990, theorem 8.1).
+__device__ __forceinline__ double quotient(double a, double b, double r) {
+    const double q = a * r;
+    return fma(fma(-q, b, a), r, q);
+}
+
+// White balance, hue, saturation and grading of one pixel (src/render.rs:3120-3180).
+__device__ __forceinline__ void colour_steps(const Chain& C, double& cr, double& cg, double& cb) {
     const lum_tonemap_params& P = C.p;
-    uint32_t i = 0, j = 0;
-    if (P.vignette > 0.0 || P.dither) {
-        j = p / w;
-        i = p - j * w;
-    }
-    double vf = 1.0;
-    if (P.vignette > 0.0) {
-        const double cx = ((double)i + 0.5) / (double)w - 0.5, cy = ((double)j + 0.5) / (double)h - 0.5;
-        vf = fmax(1.0 - (cx * cx + cy * cy) * P.vignette * 4.0, 0.0);
-    }
-    double cr = r * exposure * vf, cg = g * exposure * vf, cb = b * exposure * vf;
     if (C.wb) {
-        cr *= 1.0 + P.white_balance * 0.1;
-        cb *= 1.0 - P.white_balance * 0.1;
-        cg *= 1.0 + P.white_balance * 0.02;
+        cr *= C.wb_r;
+        cb *= C.wb_b;
+        cg *= C.wb_g;
     }
     if (C.hue) {   // rotation about the grey axis (Rodrigues)
-        const double k = 1.0 / 3.0, s3 = 1.0 / sqrt(3.0), ca = C.cos_h, sa = C.sin_h;
-        const double d = ca + k * (1.0 - ca), m = k * (1.0 - ca) - s3 * sa, p = k * (1.0 - ca) + s3 * sa;
+        const double d = C.hue_d, m = C.hue_m, p = C.hue_p;
         const double nr = cr * d + cg * m + cb * p;
         const double ng = cr * p + cg * d + cb * m;
         const double nb = cr * m + cg * p + cb * d;
@@ -181,6 +180,51 @@ __device__ __noinline__ uint32_t pixel_full(const Chain& C, double r, double g, 
         cg *= P.grade_shadows[1] * (1.0 - t) + P.grade_highlights[1] * t;
         cb *= P.grade_shadows[2] * (1.0 - t) + P.grade_highlights[2] * t;
     }
+}
+
+// The steps on quantised bytes (src/render.rs:3200-3260): brightness and contrast, then sepia across
+// the channels, then tint, colour balance and posterise.
+__device__ __forceinline__ uint32_t byte_before(const Chain& C, uint32_t v) {
+    if (C.bright) v = (uint32_t)min(max((int)v + (int)C.bright_off, 0), 255);
+    if (C.contrast) v = sat_u8(fmin(fmax((((double)v / 255.0 - 0.5) * C.p.contrast + 0.5) * 255.0, 0.0), 255.0));
+    return v;
+}
+__device__ __forceinline__ void sepia(double s, uint32_t& R, uint32_t& G, uint32_t& B) {
+    const double fr = R / 255.0, fg = G / 255.0, fb = B / 255.0;
+    const double sr = fmin(fr * 0.393 + fg * 0.769 + fb * 0.189, 1.0);
+    const double sg = fmin(fr * 0.349 + fg * 0.686 + fb * 0.168, 1.0);
+    const double sb = fmin(fr * 0.272 + fg * 0.534 + fb * 0.131, 1.0);
+    R = sat_u8((fr * (1.0 - s) + sr * s) * 255.0);
+    G = sat_u8((fg * (1.0 - s) + sg * s) * 255.0);
+    B = sat_u8((fb * (1.0 - s) + sb * s) * 255.0);
+}
+__device__ __forceinline__ uint32_t byte_after(const Chain& C, int c, uint32_t v) {
+    const lum_tonemap_params& P = C.p;
+    if (C.tint) v = sat_u8(fmin(fmax((v / 255.0 * P.tint[c]) * 255.0, 0.0), 255.0));
+    if (C.balance) v = sat_u8(fmin(fmax(v * P.color_balance[c], 0.0), 255.0));
+    if (P.posterize >= 2) {
+        const double L = (double)P.posterize;
+        v = sat_u8(fmin(fmax(round((v / 255.0) * (L - 1.0)) / (L - 1.0) * 255.0, 0.0), 255.0));
+    }
+    return v;
+}
+
+// One pixel of the full chain (src/render.rs:3100-3260); pixel p = j * w + i of the output.
+__device__ __noinline__ uint32_t pixel_full(const Chain& C, double r, double g, double b, uint32_t p, uint32_t w,
+                                            uint32_t h, double exposure) {
+    const lum_tonemap_params& P = C.p;
+    uint32_t i = 0, j = 0;
+    if (P.vignette > 0.0 || P.dither) {
+        j = p / w;
+        i = p - j * w;
+    }
+    double vf = 1.0;
+    if (P.vignette > 0.0) {
+        const double cx = ((double)i + 0.5) / (double)w - 0.5, cy = ((double)j + 0.5) / (double)h - 0.5;
+        vf = fmax(1.0 - (cx * cx + cy * cy) * P.vignette * 4.0, 0.0);
+    }
+    double cr = r * exposure * vf, cg = g * exposure * vf, cb = b * exposure * vf;
+    colour_steps(C, cr, cg, cb);
     double dither = 0.0;
     if (P.dither) {   // 4x4 Bayer matrix (src/render.rs:3187-3195), (value - 0.5) / 255
         const uint64_t bayer = 0x5D7F91B36E4CA280ull;   // rows {0,8,2,10} {12,4,14,6} {3,11,1,9} {15,7,13,5}
@@ -189,43 +233,13 @@ __device__ __noinline__ uint32_t pixel_full(const Chain& C, double r, double g, 
     }
     uint32_t R = tone_gamma(P.tone_map, cr, P.gamma, dither), G = tone_gamma(P.tone_map, cg, P.gamma, dither),
              B = tone_gamma(P.tone_map, cb, P.gamma, dither);
-    if (C.bright) {
-        R = (uint32_t)min(max((int)R + (int)C.bright_off, 0), 255);
-        G = (uint32_t)min(max((int)G + (int)C.bright_off, 0), 255);
-        B = (uint32_t)min(max((int)B + (int)C.bright_off, 0), 255);
-    }
-    if (C.contrast) {
-        auto con = [&](uint32_t v) { return sat_u8(fmin(fmax((((double)v / 255.0 - 0.5) * P.contrast + 0.5) * 255.0, 0.0), 255.0)); };
-        R = con(R);
-        G = con(G);
-        B = con(B);
-    }
-    if (C.sepia) {
-        const double fr = R / 255.0, fg = G / 255.0, fb = B / 255.0, s = P.sepia;
-        const double sr = fmin(fr * 0.393 + fg * 0.769 + fb * 0.189, 1.0);
-        const double sg = fmin(fr * 0.349 + fg * 0.686 + fb * 0.168, 1.0);
-        const double sb = fmin(fr * 0.272 + fg * 0.534 + fb * 0.131, 1.0);
-        R = sat_u8((fr * (1.0 - s) + sr * s) * 255.0);
-        G = sat_u8((fg * (1.0 - s) + sg * s) * 255.0);
-        B = sat_u8((fb * (1.0 - s) + sb * s) * 255.0);
-    }
-    if (C.tint) {
-        R = sat_u8(fmin(fmax((R / 255.0 * P.tint[0]) * 255.0, 0.0), 255.0));
-        G = sat_u8(fmin(fmax((G / 255.0 * P.tint[1]) * 255.0, 0.0), 255.0));
-        B = sat_u8(fmin(fmax((B / 255.0 * P.tint[2]) * 255.0, 0.0), 255.0));
-    }
-    if (C.balance) {
-        R = sat_u8(fmin(fmax(R * P.color_balance[0], 0.0), 255.0));
-        G = sat_u8(fmin(fmax(G * P.color_balance[1], 0.0), 255.0));
-        B = sat_u8(fmin(fmax(B * P.color_balance[2], 0.0), 255.0));
-    }
-    if (P.posterize >= 2) {
-        const double L = (double)P.posterize;
-        auto post = [&](uint32_t v) { return sat_u8(fmin(fmax(round((v / 255.0) * (L - 1.0)) / (L - 1.0) * 255.0, 0.0), 255.0)); };
-        R = post(R);
-        G = post(G);
-        B = post(B);
-    }
+    R = byte_before(C, R);
+    G = byte_before(C, G);
+    B = byte_before(C, B);
+    if (C.sepia) sepia(P.sepia, R, G, B);
+    R = byte_after(C, 0, R);
+    G = byte_after(C, 1, G);
+    B = byte_after(C, 2, B);
     return R | (G << 8) | (B << 16) | (255u << 24);
 }
 
@@ -366,9 +380,23 @@ __global__ void __launch_bounds__(kLogThreads) k_loglum(const float* __restrict_
     if constexpr (VEC) {
         const float4* in = reinterpret_cast<const float4*>(hdr);
         const uint32_t n4 = n / 4;
-        for (uint32_t q = t0; q < n4; q += stride) {
-            const float4 a = in[3 * q], b = in[3 * q + 1], c = in[3 * q + 2];
-            acc += (log_lum(a.x, a.y, a.z) + log_lum(a.w, b.x, b.y)) + (log_lum(b.z, b.w, c.x) + log_lum(c.y, c.z, c.w));
+        // kLogAhead steps' loads at once (the 256 blocks leave a third of the SMs one block each, so
+        // a step's latency counts): 4K with auto-exposure, 1 / 2 / 4 / 8 steps 67.5 / 64.3 / 61.6 /
+        // 60.7 us.  The sums stay in the order of one step after another.
+        for (uint64_t q = t0; q < n4; q += (uint64_t)kLogAhead * stride) {
+            float4 f[kLogAhead][3];
+#pragma unroll
+            for (int k = 0; k < kLogAhead; ++k) {
+                const uint64_t p = q + (uint64_t)k * stride;
+                if (p < n4)
+                    for (int j = 0; j < 3; ++j) f[k][j] = in[3 * p + j];
+            }
+#pragma unroll
+            for (int k = 0; k < kLogAhead; ++k) {
+                const float4 a = f[k][0], b = f[k][1], c = f[k][2];
+                if (q + (uint64_t)k * stride < n4)
+                    acc += (log_lum(a.x, a.y, a.z) + log_lum(a.w, b.x, b.y)) + (log_lum(b.z, b.w, c.x) + log_lum(c.y, c.z, c.w));
+            }
         }
         from = 4 * n4;
     }
@@ -566,12 +594,100 @@ __global__ void __launch_bounds__(kFlatThreads, kFlatBlocks) k_tonemap_flat(cons
     }
 }
 
+// Chains with optional steps other than dither: one pixel per lane and tile of 32, its colour steps
+// in f64 as in pixel_full, each channel's byte from the byte table (shared memory), the steps on
+// bytes from tables of the 256 bytes that each block fills first.  pixel_full evaluated the curve and
+// the power per channel and six divisions per pixel, and was bound by instruction fetch (5.6 stalled
+// warps per issue): 1080p with auto-exposure, grading, vignette and contrast 140 -> 40 us with
+// k_loglum (25 MB twice: 8 us at the copy rate; the f64 steps bound it now).  3 / 4 / 5 / 6 blocks/SM
+// 39.9 / 41.0 / 43.1 / 43.1 us.
+constexpr int kGradedThreads = 256;
+constexpr int kGradedBlocks = 3;
+template <int KIND>
+__global__ void __launch_bounds__(kGradedThreads, kGradedBlocks)
+    k_tonemap_graded(const float* __restrict__ hdr, uint32_t w, uint32_t h, const __grid_constant__ Chain C, double exposure,
+                     const double* __restrict__ partials, uint8_t* __restrict__ rgba, const ByteTable T) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ uint8_t s_before[256], s_after[3][256];
+    __shared__ float s_px[kGradedThreads / 32][96];
+    auto* tab = reinterpret_cast<unsigned long long*>(s_raw);
+    const int top = T.nb + 1;
+    for (int i = threadIdx.x; i <= top; i += kGradedThreads) tab[i] = __ldg(T.tab + i);
+    static_assert(kGradedThreads == 256, "one byte per thread");
+    s_before[threadIdx.x] = (uint8_t)byte_before(C, threadIdx.x);
+    for (int c = 0; c < 3; ++c) s_after[c][threadIdx.x] = (uint8_t)byte_after(C, c, threadIdx.x);
+    const uint32_t n = w * h;
+    if (partials) exposure = auto_exposure(partials, n, exposure);
+    __syncthreads();
+    const lum_tonemap_params& P = C.p;
+    auto byte_of = [&](double x) -> uint32_t {
+        if (!(x < 1e30)) {   // NaN (byte 0) and x beyond the table's range
+            const double q64 = x != x ? -1.0 : tone_gamma64(KIND, x, P.gamma, 0.0);
+            return q64 < 0.0 ? 0u : sat_u8(q64);
+        }
+        const long long b = __double_as_longlong(x);   // zero and negatives come before entry 1: byte 0
+        const unsigned long long e = tab[min(max((int)(b >> kTabShift) - (int)T.k0 + 1, 0), top)];
+        return (uint32_t)(e >> 56) + (((unsigned long long)b & kTabLowMask) >= (e & (2ull * kTabLowMask + 1ull)) ? 1u : 0u);
+    };
+    const int lane = threadIdx.x & 31;
+    float* px = s_px[threadIdx.x >> 5];
+    const double dw = (double)w, dh = (double)h, rw = 1.0 / dw, rh = 1.0 / dh;
+    const uint32_t tiles = (n + 31) / 32, step = gridDim.x * (kGradedThreads / 32), lim = 3 * (n / 4);
+    const float4* in = reinterpret_cast<const float4*>(hdr);
+    auto fetch = [&](uint32_t t) {
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t >= tiles || lane >= 24) return f;
+        const uint32_t i = 24 * t + lane;
+        if (i < lim) return __ldcs(in + i);
+        const uint64_t k = 4 * (uint64_t)i, end = 3 * (uint64_t)n;   // the last n % 4 pixels
+        if (k < end) f.x = hdr[k];
+        if (k + 1 < end) f.y = hdr[k + 1];
+        if (k + 2 < end) f.z = hdr[k + 2];
+        if (k + 3 < end) f.w = hdr[k + 3];
+        return f;
+    };
+    uint32_t t = blockIdx.x * (kGradedThreads / 32) + (threadIdx.x >> 5);
+    float4 f = fetch(t);
+    for (; t < tiles; t += step) {
+        if (lane < 24) reinterpret_cast<float4*>(px)[lane] = f;
+        if (t < tiles - min(tiles, step)) f = fetch(t + step);
+        __syncwarp();
+        const double r = px[3 * lane], g = px[3 * lane + 1], b = px[3 * lane + 2];
+        __syncwarp();
+        const uint32_t p = 32 * t + lane;
+        double cr = r * exposure, cg = g * exposure, cb = b * exposure;
+        if (P.vignette > 0.0) {
+            const uint32_t j = p / w, i = p - j * w;
+            const double cx = quotient((double)i + 0.5, dw, rw) - 0.5, cy = quotient((double)j + 0.5, dh, rh) - 0.5;
+            const double vf = fmax(1.0 - (cx * cx + cy * cy) * P.vignette * 4.0, 0.0);
+            cr *= vf;
+            cg *= vf;
+            cb *= vf;
+        }
+        colour_steps(C, cr, cg, cb);
+        uint32_t R = s_before[byte_of(cr)], G = s_before[byte_of(cg)], B = s_before[byte_of(cb)];
+        if (C.sepia) sepia(P.sepia, R, G, B);
+        if (p < n)
+            __stcs(reinterpret_cast<uint32_t*>(rgba) + p,
+                   s_after[0][R] | ((uint32_t)s_after[1][G] << 8) | ((uint32_t)s_after[2][B] << 16) | 0xFF000000u);
+    }
+}
+
 Chain make_chain(const lum_tonemap_params& p) {
     Chain C;
     C.p = p;
     const double ang = p.hue_shift * (3.14159265358979323846 / 180.0);
     C.cos_h = std::cos(ang);
     C.sin_h = std::sin(ang);
+    {
+        const double k = 1.0 / 3.0, s3 = 1.0 / std::sqrt(3.0), ca = C.cos_h, sa = C.sin_h;
+        C.hue_d = ca + k * (1.0 - ca);
+        C.hue_m = k * (1.0 - ca) - s3 * sa;
+        C.hue_p = k * (1.0 - ca) + s3 * sa;
+    }
+    C.wb_r = 1.0 + p.white_balance * 0.1;
+    C.wb_g = 1.0 + p.white_balance * 0.02;
+    C.wb_b = 1.0 - p.white_balance * 0.1;
     double bo = p.brightness * 255.0;
     bo = bo != bo ? 0.0 : (bo > 32767.0 ? 32767.0 : (bo < -32768.0 ? -32768.0 : bo));
     C.bright_off = (int16_t)bo;
@@ -716,6 +832,7 @@ cudaError_t launch_tonemap(const float* hdr, uint32_t w, uint32_t h, const lum_t
     }
     const tone::Chain C = tone::make_chain(tm);
     const tone::ByteTable T = C.extra ? tone::ByteTable{nullptr, nullptr, 0, 0} : tone::byte_table(tm.tone_map, tm.gamma);
+    const tone::ByteTable G = C.extra && !tm.dither ? tone::byte_table(tm.tone_map, tm.gamma) : tone::ByteTable{nullptr, nullptr, 0, 0};
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -741,6 +858,13 @@ cudaError_t launch_tonemap(const float* hdr, uint32_t w, uint32_t h, const lum_t
             else
                 tone::k_tonemap_flat<K, false><<<fg, tone::kFlatThreads, 8 * ents, stream>>>(hdr, (uint32_t)n, 0, exposure, partials,
                                                                                             rgba, T, C.inv_gamma);
+            return;
+        }
+        if (vec && C.extra && !tm.dither && G.tab) {
+            const size_t warps = (n + 31) / 32;
+            const int gg = (int)std::max<size_t>(1, std::min<size_t>((warps + 7) / 8, (size_t)nsm * tone::kGradedBlocks));
+            tone::k_tonemap_graded<K><<<gg, tone::kGradedThreads, 8 * ((size_t)G.nb + 2), stream>>>(
+                hdr, (uint32_t)w, (uint32_t)h, C, exposure, partials, rgba, G);
             return;
         }
         if (vec)

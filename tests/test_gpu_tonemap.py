@@ -137,3 +137,26 @@ def test_common_chain_over_tiles_and_rare_values(curve, exposure):
         torch.cuda.synchronize()
         with np.errstate(all="ignore"):
             compare(d_out.cpu().numpy(), OT.tonemap(img, chain))
+
+
+@pytest.mark.parametrize("chain", [
+    {"saturation": 1.3, "vignette": 0.5}, {"hue_shift": 30.0, "contrast": 1.3, "brightness": -0.1, "gamma": 2.2},
+    {"tone_map": OT.REINHARD, "sepia": 0.6, "posterize": 5, "white_balance": -0.7},
+    {"tone_map": OT.NONE, "tint": (0.9, 1.0, 0.7), "color_balance": (1.2, 0.9, 1.0), "auto_exposure": True,
+     "grade_shadows": (0.8, 1.0, 1.2), "grade_highlights": (1.1, 1.0, 0.9)}])
+def test_graded_chain_over_ragged_tiles_and_rare_values(chain):
+    """The optional steps at widths and pixel counts around the 32-pixel tiles, with zeros, negatives,
+    huge values and NaN among the pixels (infinities would make the auto-exposure's mean infinite)."""
+    import torch
+    rare = np.array([0.0, -0.0, -1.0, 1e-45, 1e30, 3e37, np.nan, 1e20], np.float32)
+    for w, h in ((1, 1), (1, 33), (31, 1), (5, 13), (64, 3), (127, 9)):
+        img = hdr_image(h, w, w * h)
+        if not chain.get("auto_exposure"):
+            flat = img.reshape(-1)
+            flat[::11][: len(rare)] = rare[: len(flat[::11])]
+        d_hdr, d_out = torch.from_numpy(img).cuda(), torch.zeros((h, w, 4), dtype=torch.uint8, device="cuda")
+        scratch = torch.empty(abi.TONEMAP_SCRATCH_BYTES, dtype=torch.uint8, device="cuda")
+        L.tonemap_device(d_hdr.data_ptr(), w, h, tm_config(chain), scratch.data_ptr(), d_out.data_ptr())
+        torch.cuda.synchronize()
+        with np.errstate(all="ignore"):
+            compare(d_out.cpu().numpy(), OT.tonemap(img, chain))
