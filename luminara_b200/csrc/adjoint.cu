@@ -553,7 +553,7 @@ __device__ void sweep_path(const SceneDev& S, const RenderDev& R, const PathHead
 }
 
 #ifndef LUM_ADJ_MIN_BLOCKS
-#define LUM_ADJ_MIN_BLOCKS 5
+#define LUM_ADJ_MIN_BLOCKS 6
 #endif
 
 constexpr uint32_t kReplayStrata = 8;   // strata per replay task (tile x stratum group)
@@ -571,7 +571,8 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                                                                   float* __restrict__ inv_wsum_px, WorkCounters* wc) {
     extern __shared__ int smem_raw[];
     int* stack = lane_stack(smem_raw);
-    const int lane = threadIdx.x & 31;
+    __shared__ uint32_t s_slot[4][32], s_next[4];   // per warp: pixels to replay, next pair of the pool
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t err = 0;
     const uint32_t n_st = R.s_end - R.s_begin;
     const uint32_t n_groups = (n_st + kReplayStrata - 1) / kReplayStrata;
@@ -587,16 +588,15 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
         const uint32_t i = (tile % R.tiles_x) * 8 + (lane & 7);
         const uint32_t j = (tile / R.tiles_x) * 4 + (lane >> 3);
         const bool valid = i < R.w && j < R.h;
-        const uint32_t gi = i + R.crop_x, gj = j + R.crop_y;
-        const uint32_t pixel = gj * R.full_w + gi;
-        const size_t slot_base = (size_t)(tile - t0) * n_st * 32 + lane;
-        uint32_t st = s_hi;
+        const size_t slot_base = (size_t)(tile - t0) * n_st * 32;
+        bool replay = false;                            // the pixel has a gradient
         if (valid) {
             const float* g = dldi + 3 * ((size_t)j * R.w + i);
-            if (g[0] != 0.0f || g[1] != 0.0f || g[2] != 0.0f) st = s_lo;
+            replay = g[0] != 0.0f || g[1] != 0.0f || g[2] != 0.0f;
         }
         if (valid && group == 0) {
             // pixel = sum_s f(L_s) w_s / sum_s w_s (render.rs:1699-1705)
+            const uint32_t pixel = (j + R.crop_y) * R.full_w + i + R.crop_x;
             float wsum = 0.0f;
             if (R.pixel_filter == LUM_FILTER_BOX) {
                 wsum = (float)n_st;
@@ -611,10 +611,17 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
             }
             inv_wsum_px[(size_t)j * R.w + i] = wsum > 0.0f ? 1.0f / wsum : 1.0f;
         }
-        if (st == s_hi)                                 // nothing to replay for this lane
-            for (uint32_t s2 = s_lo; s2 < s_hi; ++s2) heads[slot_base + (size_t)(s2 - R.s_begin) * 32].K = -1;
+        if (!replay)                                    // nothing to replay for this pixel
+            for (uint32_t s2 = s_lo; s2 < s_hi; ++s2) heads[slot_base + lane + (size_t)(s2 - R.s_begin) * 32].K = -1;
+        const unsigned with = __ballot_sync(kFullMask, replay);
+        const uint32_t n_px = __popc(with), n_items = n_px * (s_hi - s_lo);
+        // idx / n_px by a high multiply (idx * n_px < 2^32); 0: one pixel
+        const uint32_t magic = n_px > 1 ? 0xFFFFFFFFu / n_px + 1u : 0u;
+        if (replay) s_slot[wid][__popc(with & ((1u << lane) - 1u))] = lane;
+        if (lane == 0) s_next[wid] = 0u;
+        __syncwarp(kFullMask);
         int state = A_IDLE;
-        uint32_t cur = 0;
+        uint32_t cur = 0, px = 0, pixel = 0;
         int K = 0;
         uint32_t vflags = 0;
         float vsp = 0.0f;
@@ -625,15 +632,23 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
         Trav tv;                // place of a suspended walk
         bool found = false, walking = false;
         for (;;) {
-            if (state == A_IDLE && st < s_hi) {
-                start_path<philox_unroll<CLS>()>(S, R, gi, gj, pixel, st, P);
-                cur = st++;
-                K = 0;
-                bg = mk(0.f, 0.f, 0.f);
-                state = R.max_depth > 0 ? A_CLOSEST : A_DONE;
+            if (state == A_IDLE) {
+                const uint32_t idx = atomicAdd(&s_next[wid], 1u);
+                if (idx < n_items) {
+                    const uint32_t k = magic ? __umulhi(idx, magic) : idx;
+                    px = s_slot[wid][idx - k * n_px];
+                    cur = s_lo + k;
+                    const uint32_t gi = (tile % R.tiles_x) * 8 + (px & 7) + R.crop_x;
+                    const uint32_t gj = (tile / R.tiles_x) * 4 + (px >> 3) + R.crop_y;
+                    pixel = gj * R.full_w + gi;
+                    start_path<philox_unroll<CLS>()>(S, R, gi, gj, pixel, cur, P);
+                    K = 0;
+                    bg = mk(0.f, 0.f, 0.f);
+                    state = R.max_depth > 0 ? A_CLOSEST : A_DONE;
+                }
             }
             if (!__any_sync(kFullMask, state != A_IDLE)) break;
-            const size_t slot = slot_base + (size_t)(cur - R.s_begin) * 32;
+            const size_t slot = slot_base + px + (size_t)(cur - R.s_begin) * 32;
             {
                 const bool shadow = state == A_SHADOW, act = shadow || state == A_CLOSEST;
                 Ray r;
@@ -700,7 +715,7 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                 ph.jy = P.jy;
                 ph.K = K;
                 ph.pixel = pixel;
-                ph.local = j * R.w + i;
+                ph.local = ((tile / R.tiles_x) * 4 + (px >> 3)) * R.w + (tile % R.tiles_x) * 8 + (px & 7);
                 ph.st = cur;
                 heads[slot] = ph;
                 state = A_IDLE;
@@ -838,7 +853,7 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
         int nsm = 0, devi = 0;
         cudaGetDevice(&devi);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, devi);
-        const size_t stack = stack_smem(kStackDepth, 128);
+        const size_t stack = stack_smem(dev.stack_depth, 128);   // sized to the scene's BVH
         auto replay = dev.cls == CLS_QUAD ? adj::k_replay<CLS_QUAD>
                     : dev.cls == CLS_MESH ? adj::k_replay<CLS_MESH> : adj::k_replay<CLS_ALL>;
         int occ_r = 0;
