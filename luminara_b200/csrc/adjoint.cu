@@ -560,7 +560,10 @@ __device__ __forceinline__ void sweep_vertex(const SceneDev& S, const RenderDev&
 #define LUM_ADJ_MIN_BLOCKS 6
 #endif
 
-constexpr uint32_t kReplayStrata = 8;   // strata per replay task (tile x stratum group)
+// Strata per replay task (tile x stratum group): 8, fewer (4, 2) while the launch would otherwise have
+// less than kReplayTasks tasks per resident warp -- a task ends with its slowest path, but warps
+// without a task idle.  512x512 quads 64 spp 8 / 4 strata: kernels 13.4 / 14.1 ms; 133x77 16 spp 0.79 / 0.52.
+constexpr uint32_t kReplayStrata = 8, kReplayTasks = 4;
 
 // Replay kernel: the forward megakernel's state machine (same functions, same RNG keys, one
 // traversal per loop iteration for every tracing lane) over the tiles [t0, t1), a task being
@@ -572,14 +575,15 @@ template <int CLS>
 __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, RenderDev R, const float* __restrict__ dldi,
                                                                   uint32_t t0, uint32_t t1, PathHead* __restrict__ heads,
                                                                   Vert* __restrict__ verts, size_t n_slots,
-                                                                  float* __restrict__ inv_wsum_px, WorkCounters* wc) {
+                                                                  float* __restrict__ inv_wsum_px, WorkCounters* wc,
+                                                                  uint32_t task_strata) {
     extern __shared__ int smem_raw[];
     int* stack = lane_stack(smem_raw);
     __shared__ uint32_t s_slot[4][32], s_next[4];   // per warp: pixels to replay, next pair of the pool
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t err = 0;
     const uint32_t n_st = R.s_end - R.s_begin;
-    const uint32_t n_groups = (n_st + kReplayStrata - 1) / kReplayStrata;
+    const uint32_t n_groups = (n_st + task_strata - 1) / task_strata;
     const uint32_t n_tasks = (t1 - t0) * n_groups;
     enum : int { A_IDLE = 0, A_CLOSEST = 1, A_SHADOW = 2, A_DONE = 3 };
     for (;;) {
@@ -588,7 +592,7 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
         task = __shfl_sync(kFullMask, task, 0);
         if (task >= n_tasks) break;
         const uint32_t tile = t0 + task / n_groups, group = task % n_groups;
-        const uint32_t s_lo = R.s_begin + group * kReplayStrata, s_hi = min(R.s_end, s_lo + kReplayStrata);
+        const uint32_t s_lo = R.s_begin + group * task_strata, s_hi = min(R.s_end, s_lo + task_strata);
         const uint32_t i = (tile % R.tiles_x) * 8 + (lane & 7);
         const uint32_t j = (tile / R.tiles_x) * 4 + (lane >> 3);
         const bool valid = i < R.w && j < R.h;
@@ -824,6 +828,9 @@ __global__ void __launch_bounds__(kSweepThreads, 5) k_sweep(SceneDev S, RenderDe
 
 namespace {
 
+// Vertex staging of one chunk: within what the pool keeps for reuse, with room for the scenes.
+constexpr size_t kStagingBytes = (size_t)3584 << 20;
+
 lum_status adj_cuda(cudaError_t e, const char* what) {
     char msg[256];
     snprintf(msg, sizeof msg, "%s: %s", what, cudaGetErrorString(e));
@@ -870,12 +877,14 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
     std::memset(d_emission, 0, sizeof(float) * 3 * n_mat);
     if (px == 0 || R.s_end <= R.s_begin || n_mat == 0 || R.max_depth == 0) return LUM_OK;
     // Paths are replayed a chunk of tiles at a time into a staging buffer of vertex records
-    // (bounded, at most 8 GiB or a quarter of free device memory), then swept.
+    // (bounded, at most kStagingBytes or a quarter of free device memory), then swept.  The buffer
+    // comes from the scenes' pool and goes back to it: allocating and freeing 7.2 GB took 5-20 ms per
+    // call on B200.
     const uint32_t n_st = R.s_end - R.s_begin;
     const size_t per_tile = (size_t)32 * n_st * (sizeof(adj::PathHead) + (size_t)R.max_depth * sizeof(adj::Vert));
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    const size_t budget = std::max<size_t>(per_tile, std::min<size_t>((size_t)8 << 30, free_b / 4));
+    const size_t budget = std::max<size_t>(per_tile, std::min<size_t>(kStagingBytes, free_b / 4));
     const uint32_t chunk_tiles = (uint32_t)std::min<size_t>(R.n_tasks, budget / per_tile);
     const size_t n_slots = (size_t)chunk_tiles * 32 * n_st;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -887,8 +896,8 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
                  o_heads = o_wc + al(sizeof(WorkCounters)), o_verts = o_heads + al(bytes_heads),
                  total = o_verts + al(bytes_verts);
     char* buf = nullptr;
-    cudaError_t e = cudaMalloc(&buf, total);
-    if (e != cudaSuccess) return adj_cuda(e, "cudaMalloc");
+    if ((st = scratch_alloc(scene, (void**)&buf, total)) != LUM_OK) return st;
+    cudaError_t e = cudaSuccess;
     float* d_img = (float*)buf;
     float* d_g = (float*)(buf + o_g);
     int* d_lm = (int*)(buf + o_lm);
@@ -936,7 +945,10 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
             cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s);
         int occ_s = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, sweep, adj::kSweepThreads, smem_s);
-        const uint32_t n_groups = (n_st + adj::kReplayStrata - 1) / adj::kReplayStrata;
+        uint32_t task_strata = adj::kReplayStrata;
+        const size_t want = (size_t)adj::kReplayTasks * nsm * std::max(occ_r, 1) * 4;
+        while (task_strata > 2 && (size_t)chunk_tiles * ((n_st + task_strata - 1) / task_strata) < want) task_strata /= 2;
+        const uint32_t n_groups = (n_st + task_strata - 1) / task_strata;
         const int grid_r = (int)std::min<size_t>((size_t)nsm * std::max(occ_r, 1), ((size_t)chunk_tiles * n_groups + 3) / 4);
         const int grid_s = (int)std::min<size_t>((size_t)nsm * std::max(occ_s, 1), (n_slots + 4 * window - 1) / (4 * window));
         cudaEventRecord(ev0, stream);
@@ -945,7 +957,8 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
             const size_t slots = (size_t)(c1 - c0) * 32 * n_st;
             e = cudaMemsetAsync(&wc->next_task, 0, sizeof(uint32_t), stream);
             if (e == cudaSuccess) {
-                replay<<<grid_r, 128, stack, stream>>>(dev, R, d_img, c0, c1, d_heads, d_verts, n_slots, d_ws, wc);
+                replay<<<grid_r, 128, stack, stream>>>(dev, R, d_img, c0, c1, d_heads, d_verts, n_slots, d_ws, wc,
+                                                        task_strata);
                 e = cudaGetLastError();
             }
             if (e == cudaSuccess) {
@@ -966,7 +979,7 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
     if (ok) cudaEventElapsedTime(&ms, ev0, ev1);
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
-    cudaFree(buf);
+    scratch_free(scene, buf);
     if (!ok) return adj_cuda(e, "lum_backward");
     std::memcpy(d_albedo, hg.data(), sizeof(float) * 3 * n_mat);
     std::memcpy(d_roughness, hg.data() + 3 * n_mat, sizeof(float) * n_mat);

@@ -678,12 +678,15 @@ lum_status ensure(lum_scene* s, void** ptr, size_t* cap, size_t bytes) {
     return LUM_OK;
 }
 
-// Readback of a device buffer into pageable host memory through two pinned staging chunks: the
-// copy engine fills one chunk while host threads copy the other into place.  A direct
-// cudaMemcpy into pageable memory took 1.4-6.3 ms for a 25 MB frame on the B200 box, a copy into
-// pinned memory 0.46 ms.  The staging buffers are per device and shared; a readback that finds
-// them busy (another thread's) copies directly.
-constexpr size_t kStageChunk = 4u << 20;
+// Transfers between pageable host memory and the device through two pinned staging chunks: the
+// copy engine moves one chunk while host threads copy the other.  A direct cudaMemcpy into
+// pageable memory took 1.4-6.3 ms for a 25 MB frame on the B200 box, a copy into pinned memory
+// 0.46 ms.  A million rays up and their hits down (88 MB) 14.1 -> 4.5 ms with 8 MB chunks and 16
+// threads (4 MB and 8 threads 5.7), full HD AOVs (21 MB) 1.66 -> 1.04 ms with 2 MB and 4.  The staging buffers are per device and shared; a call that finds them busy (another
+// thread's) copies directly, as do transfers below kStageMin, where the driver's own path is
+// as fast.
+constexpr size_t kStageChunk = 8u << 20;
+constexpr size_t kStageMin = 1u << 20;
 
 struct Staging {
     std::mutex mu;
@@ -696,46 +699,110 @@ Staging* staging(int dev) {
     return dev >= 0 && dev < kPoolDevices ? &st[dev] : nullptr;
 }
 
+// Two team sizes only: libgomp rebuilds its team when the size changes.
 void host_copy(unsigned char* dst, const unsigned char* src, size_t n) {
-    constexpr size_t kSlice = 256u << 10;
-    const long slices = (long)((n + kSlice - 1) / kSlice);
-    const int nt = std::max(1, std::min({8, omp_get_num_procs(), (int)slices}));
+    const int nt = std::max(1, std::min(n > (3u << 20) ? 16 : 4, omp_get_num_procs()));
+    const size_t slice = (n / nt + 4095) & ~(size_t)4095;
 #pragma omp parallel for num_threads(nt) schedule(static)
-    for (long k = 0; k < slices; ++k) {
-        const size_t o = (size_t)k * kSlice;
-        std::memcpy(dst + o, src + o, std::min(kSlice, n - o));
+    for (int k = 0; k < nt; ++k) {
+        const size_t o = (size_t)k * slice;
+        if (o < n) std::memcpy(dst + o, src + o, k == nt - 1 ? n - o : std::min(slice, n - o));
     }
 }
 
-lum_status readback(lum_scene* s, void* dst, const void* src, size_t bytes, cudaStream_t stream) {
-    Staging* sg = staging(s->device);
-    std::unique_lock<std::mutex> lk;
-    if (sg) lk = std::unique_lock<std::mutex>(sg->mu, std::try_to_lock);
-    if (bytes < 2 * kStageChunk || !sg || !lk.owns_lock()) {
-        CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync D2H");
-        CU(cudaStreamSynchronize(stream), "D2H");
+// One call's transfers on one stream: holds the staging buffers (if they are free) until the call
+// ends, with no copy of theirs in flight.
+class Transfers {
+public:
+    Transfers(int device, cudaStream_t stream) : stream_(stream), sg_(staging(device)) {
+        if (sg_) lk_ = std::unique_lock<std::mutex>(sg_->mu, std::try_to_lock);
+        if (!lk_.owns_lock()) sg_ = nullptr;
+    }
+    ~Transfers() {
+        if (pending_) cudaStreamSynchronize(stream_);   // before another call writes the buffers
+    }
+
+    // host -> device; the source may be reused on return.
+    lum_status up(void* dst, const void* src, size_t bytes) {
+        if (!staged(bytes)) {
+            CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream_), "cudaMemcpyAsync H2D");
+            return LUM_OK;
+        }
+        lum_status st = prepare();
+        if (st != LUM_OK) return st;
+        const size_t chunk = chunk_of(bytes);
+        for (size_t o = 0; o < bytes; o += chunk) {
+            const size_t n = std::min(chunk, bytes - o);
+            const int b = next();
+            CU(cudaEventSynchronize(sg_->ev[b]), "H2D");   // the buffer's last copy has left it
+            host_copy(sg_->buf[b], static_cast<const unsigned char*>(src) + o, n);
+            CU(cudaMemcpyAsync(static_cast<unsigned char*>(dst) + o, sg_->buf[b], n, cudaMemcpyHostToDevice, stream_),
+               "cudaMemcpyAsync H2D");
+            CU(cudaEventRecord(sg_->ev[b], stream_), "cudaEventRecord");
+            pending_ = true;
+        }
         return LUM_OK;
     }
-    for (int b = 0; b < 2; ++b) {
-        if (!sg->buf[b]) CU(cudaHostAlloc((void**)&sg->buf[b], kStageChunk, cudaHostAllocPortable), "cudaHostAlloc");
-        if (!sg->ev[b]) CU(cudaEventCreateWithFlags(&sg->ev[b], cudaEventDisableTiming), "cudaEventCreate");
-    }
-    const size_t n_chunks = (bytes + kStageChunk - 1) / kStageChunk;
-    auto* d = static_cast<unsigned char*>(dst);
-    const auto* g = static_cast<const unsigned char*>(src);
-    for (size_t i = 0; i <= n_chunks; ++i) {
-        if (i < n_chunks) {   // chunk i into buffer i % 2, whose previous chunk the host has copied out
-            const size_t o = i * kStageChunk, n = std::min(kStageChunk, bytes - o);
-            CU(cudaMemcpyAsync(sg->buf[i & 1], g + o, n, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync D2H");
-            CU(cudaEventRecord(sg->ev[i & 1], stream), "cudaEventRecord");
+
+    // device -> host, waited for.
+    lum_status down(void* dst, const void* src, size_t bytes) {
+        if (!staged(bytes)) {
+            CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_), "cudaMemcpyAsync D2H");
+            CU(cudaStreamSynchronize(stream_), "D2H");
+            pending_ = false;
+            return LUM_OK;
         }
-        if (i > 0) {          // chunk i - 1 to its place
-            const size_t j = i - 1, o = j * kStageChunk, n = std::min(kStageChunk, bytes - o);
-            CU(cudaEventSynchronize(sg->ev[j & 1]), "D2H");
-            host_copy(d + o, sg->buf[j & 1], n);
+        lum_status st = prepare();
+        if (st != LUM_OK) return st;
+        const size_t chunk = chunk_of(bytes);
+        unsigned char *d = static_cast<unsigned char*>(dst), *last_dst = nullptr;
+        int last_b = 0;
+        size_t last_n = 0;
+        for (size_t o = 0;; o += chunk) {
+            const bool more = o < bytes;
+            const int b = more ? next() : 0;
+            const size_t n = more ? std::min(chunk, bytes - o) : 0;
+            if (more) {   // into the buffer whose previous chunk the host has copied out
+                CU(cudaMemcpyAsync(sg_->buf[b], static_cast<const unsigned char*>(src) + o, n, cudaMemcpyDeviceToHost,
+                                   stream_), "cudaMemcpyAsync D2H");
+                CU(cudaEventRecord(sg_->ev[b], stream_), "cudaEventRecord");
+                pending_ = true;
+            }
+            if (last_n) {   // the chunk before it to its place
+                CU(cudaEventSynchronize(sg_->ev[last_b]), "D2H");
+                host_copy(last_dst, sg_->buf[last_b], last_n);
+            }
+            if (!more) break;
+            last_dst = d + o;
+            last_b = b;
+            last_n = n;
         }
+        pending_ = false;
+        return LUM_OK;
     }
-    return LUM_OK;
+
+private:
+    bool staged(size_t bytes) const { return sg_ && bytes >= kStageMin; }
+    static size_t chunk_of(size_t bytes) {   // at least four chunks of a short transfer overlap
+        return std::min(kStageChunk, std::max((size_t)256 << 10, (bytes / 4 + 4095) & ~(size_t)4095));
+    }
+    int next() { return turn_ ^= 1; }
+    lum_status prepare() {
+        for (int b = 0; b < 2; ++b) {
+            if (!sg_->buf[b]) CU(cudaHostAlloc((void**)&sg_->buf[b], kStageChunk, cudaHostAllocPortable), "cudaHostAlloc");
+            if (!sg_->ev[b]) CU(cudaEventCreateWithFlags(&sg_->ev[b], cudaEventDisableTiming), "cudaEventCreate");
+        }
+        return LUM_OK;
+    }
+    cudaStream_t stream_;
+    Staging* sg_;
+    std::unique_lock<std::mutex> lk_;
+    int turn_ = 0;
+    bool pending_ = false;   // copies through the buffers not known to have finished
+};
+
+lum_status readback(lum_scene* s, void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+    return Transfers(s->device, stream).down(dst, src, bytes);
 }
 
 lum_status make_render_dev(const lum_scene* s, const lum_render_params& p, lum::RenderDev& R) {
@@ -1197,12 +1264,13 @@ lum_status lum_render_aov(lum_scene* s, const lum_render_params* params, float* 
     CU(cudaMemsetAsync(s->d_work, 0, sizeof(lum::WorkCounters), s->stream), "cudaMemsetAsync");
     CU(lum::launch_aov(s->dev, R, depth ? d_depth : nullptr, normals ? d_norm : nullptr, albedo ? d_alb : nullptr,
                        s->d_work, s->stream), "aov launch");
-    if (depth) CU(cudaMemcpyAsync(depth, d_depth, 4 * px, cudaMemcpyDeviceToHost, s->stream), "D2H");
-    if (normals) CU(cudaMemcpyAsync(normals, d_norm, 3 * px, cudaMemcpyDeviceToHost, s->stream), "D2H");
-    if (albedo) CU(cudaMemcpyAsync(albedo, d_alb, 3 * px, cudaMemcpyDeviceToHost, s->stream), "D2H");
     lum::WorkCounters wc{};
     CU(cudaMemcpyAsync(&wc, s->d_work, sizeof wc, cudaMemcpyDeviceToHost, s->stream), "D2H");
-    CU(cudaStreamSynchronize(s->stream), "aov");
+    Transfers tr(s->device, s->stream);
+    if (depth) st = tr.down(depth, d_depth, 4 * px);
+    if (st == LUM_OK && normals) st = tr.down(normals, d_norm, 3 * px);
+    if (st == LUM_OK && albedo) st = tr.down(albedo, d_alb, 3 * px);
+    if (st != LUM_OK) return st;
     if (wc.error_flags) return fail(LUM_ERR_KERNEL, "AOV kernel reported error flags 0x%x", wc.error_flags);
     return LUM_OK;
 }
@@ -1311,13 +1379,13 @@ lum_status lum_intersect(lum_scene* s, const lum_ray* rays, uint32_t n, lum_hit*
     if (st != LUM_OK) return st;
     lum_ray* d_r = (lum_ray*)s->d_rays;
     lum_hit* d_h = (lum_hit*)((char*)s->d_rays + rb);
-    CU(cudaMemcpyAsync(d_r, rays, sizeof(lum_ray) * (size_t)n, cudaMemcpyHostToDevice, s->stream), "H2D rays");
+    Transfers tr(s->device, s->stream);
+    if ((st = tr.up(d_r, rays, sizeof(lum_ray) * (size_t)n)) != LUM_OK) return st;
     CU(cudaMemsetAsync(s->d_work, 0, sizeof(lum::WorkCounters), s->stream), "memset");
     CU(lum::launch_intersect(s->dev, d_r, n, d_h, s->d_work, s->stream), "intersect launch");
     lum::WorkCounters wc{};
-    CU(cudaMemcpyAsync(hits, d_h, hb, cudaMemcpyDeviceToHost, s->stream), "D2H hits");
     CU(cudaMemcpyAsync(&wc, s->d_work, sizeof wc, cudaMemcpyDeviceToHost, s->stream), "D2H counters");
-    CU(cudaStreamSynchronize(s->stream), "intersect");
+    if ((st = tr.down(hits, d_h, hb)) != LUM_OK) return st;
     if (wc.error_flags) return fail(LUM_ERR_KERNEL, "intersect kernel reported error flags 0x%x", wc.error_flags);
     return LUM_OK;
 }
@@ -1332,13 +1400,13 @@ lum_status lum_occluded(lum_scene* s, const lum_ray* rays, uint32_t n, int32_t* 
     if (st != LUM_OK) return st;
     lum_ray* d_r = (lum_ray*)s->d_rays;
     int32_t* d_o = (int32_t*)((char*)s->d_rays + rb);
-    CU(cudaMemcpyAsync(d_r, rays, sizeof(lum_ray) * (size_t)n, cudaMemcpyHostToDevice, s->stream), "H2D rays");
+    Transfers tr(s->device, s->stream);
+    if ((st = tr.up(d_r, rays, sizeof(lum_ray) * (size_t)n)) != LUM_OK) return st;
     CU(cudaMemsetAsync(s->d_work, 0, sizeof(lum::WorkCounters), s->stream), "memset");
     CU(lum::launch_occluded(s->dev, d_r, n, d_o, s->d_work, s->stream), "occluded launch");
     lum::WorkCounters wc{};
-    CU(cudaMemcpyAsync(occluded, d_o, ob, cudaMemcpyDeviceToHost, s->stream), "D2H occluded");
     CU(cudaMemcpyAsync(&wc, s->d_work, sizeof wc, cudaMemcpyDeviceToHost, s->stream), "D2H counters");
-    CU(cudaStreamSynchronize(s->stream), "occluded");
+    if ((st = tr.down(occluded, d_o, ob)) != LUM_OK) return st;
     if (wc.error_flags) return fail(LUM_ERR_KERNEL, "occluded kernel reported error flags 0x%x", wc.error_flags);
     return LUM_OK;
 }
@@ -1365,6 +1433,10 @@ lum_status prepare_render(lum_scene* s, const lum_render_params* params, SceneDe
     stream = s->stream;
     return LUM_OK;
 }
+
+lum_status scratch_alloc(lum_scene* s, void** ptr, size_t bytes) { return pool_alloc(s, ptr, bytes, false); }
+
+void scratch_free(lum_scene* s, void* ptr) { cudaFreeAsync(ptr, s->stream); }
 
 int scene_max_material_kind(const lum_scene* s) { return s ? s->max_mat_kind : 0; }
 
