@@ -294,7 +294,10 @@ static int kernel_occupancy(const void* fn, size_t smem) {
 //   512x512 x 64 spp quads (8192 tiles)     2 groups of 32 strata 10.26 ms, 4 of 16  9.66 ms
 //   256x256 x 64 spp box room (2048 tiles)  7 groups of 10        1.99 ms, 14 of 5   2.02 ms,
 //                                           8 of 8                 1.94 ms
-//   128x128 x 16 spp box room (512 tiles)   4 groups of 4          0.29 ms, 2 of 8    0.43 ms
+// and since walks are warp-convergent, groups of at least 4 -> 2 strata (16 spp):
+//   128x128 quads (512 tiles) 0.504 -> 0.410 ms, 320x180 mesh (1800 tiles) 1.16 -> 0.97, 320x180
+//   spheres 0.312 -> 0.297, 128x128 box room 0.297 -> 0.292 (single strata: 0.331);
+// 16 tasks per warp, or groups of 4 strata preferred, lost 2-5% on the larger of these frames.
 // A larger frame can also split its last LUM_TAIL_TILES_PER_WARP x (resident warps) tiles into
 // LUM_TAIL_GROUPS groups, so that the launch ends on short tasks; on the 1080p frames (spheres
 // 256 spp, dense mesh 144 spp) that gained nothing -- the warps still running at the end of a
@@ -306,7 +309,7 @@ static int kernel_occupancy(const void* fn, size_t smem) {
 #define LUM_SMALL_FRAME_TASKS 8
 #endif
 #ifndef LUM_MIN_GROUP_STRATA
-#define LUM_MIN_GROUP_STRATA 4
+#define LUM_MIN_GROUP_STRATA 2
 #endif
 #ifndef LUM_PREF_GROUP_STRATA
 #define LUM_PREF_GROUP_STRATA 8
