@@ -664,7 +664,8 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                 r.o = P.ray.o;
                 r.d = shadow ? pend.dir : P.ray.d;
                 r.time = shadow ? 0.0f : P.ray.time;
-                if (act && !walking) {
+                const bool fresh = act && !walking;
+                if (fresh) {
                     h.t = shadow ? pend.tmax : CUDART_INF_F;
                     h.prim = -1;
                     h.b1 = h.b2 = 0.0f;
@@ -673,7 +674,7 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
                     found = false;
                 }
                 const bool done = walk_warp<false, false, LUM_SUSPEND_LANES, CLS>(S, r, 0.001f, shadow, h, found, tv,
-                                                                                 stack, err, act);
+                                                                                 stack, err, act, fresh);
                 walking = act && !done;
                 __syncwarp(kFullMask);   // the lanes shade together
                 if (!done) {
@@ -924,7 +925,8 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, devi);
         const size_t stack = stack_smem(dev.stack_depth, 128);   // sized to the scene's BVH
         auto replay = dev.cls == CLS_QUAD ? adj::k_replay<CLS_QUAD>
-                    : dev.cls == CLS_MESH ? adj::k_replay<CLS_MESH> : adj::k_replay<CLS_ALL>;
+                    : dev.cls == CLS_MESH ? adj::k_replay<CLS_MESH>
+                    : dev.n_big > 0 ? adj::k_replay<CLS_GROUND> : adj::k_replay<CLS_ALL>;
         int occ_r = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, replay, 128, stack);
         // Gradients accumulate per block in shared memory when the material table fits

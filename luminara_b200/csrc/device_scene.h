@@ -30,6 +30,10 @@ enum PrimType : int32_t {
 constexpr int kStackDepth = 64;     // traversal stack entries per thread
 constexpr int kMaxBlendDepth = 4;   // nesting levels of Blend materials (checked by lum_scene_create)
 constexpr int kMaxBvhDepth = 62;    // the builder keeps every leaf at most this deep
+// Spheres of at least this radius (grounds) evaluate o - c in f64 (tracer.cuh's sphere_roots); sphere
+// scenes keep up to kMaxBigSpheres of them out of the BVH.
+constexpr float kBigSphere = 32.0f;
+constexpr int kMaxBigSpheres = 4;
 constexpr int kMedianDepth = 40;    // below this depth the builder splits at the object median
 
 struct alignas(16) MatDev {
@@ -117,7 +121,7 @@ struct SceneDev {
     int32_t stack_depth;     // traversal stack entries this BVH can need (<= kStackDepth)
     int32_t moving;          // some sphere moves: camera rays draw their time
     int32_t cls;             // scene class of the general megakernel build (CLS_*, tracer.cuh)
-    int32_t pad_cls;
+    int32_t n_big;           // big spheres kept out of the BVH: primitives [n_prims - n_big, n_prims)
     const BlendEmit* blend_emit;   // emissive leaves of Blend materials
     const float* env;        // environment map, env_w * env_h RGB floats (or null)
     uint32_t env_w, env_h;

@@ -975,15 +975,35 @@ lum_status lum_scene_create(const lum_scene_desc* desc, lum_scene** out) {
     if (st != LUM_OK) return st;
     if (F.prims.size() >= (1u << 27)) return fail(LUM_ERR_TOO_LARGE, "too many primitives");
 
-    std::vector<lum::BuildBox> boxes(F.prims.size());
-    for (size_t i = 0; i < F.prims.size(); ++i) boxes[i] = F.prims[i].box;
+    // the sphere-and-basic-materials kernel class (planes are tested in the general way): static
+    // spheres (record 1's w, the moving flag, is 0)
+    bool sph = true;
+    for (size_t k = 0; k < F.prims.size() && sph; ++k)
+        sph = F.prims[k].type == lum::PT_SPHERE && F.prims[k].rec[7] == 0.0f;
+    for (uint32_t i = 0; i < desc->n_materials && sph; ++i)
+        sph = desc->materials[i].kind >= LUM_MAT_LAMBERTIAN && desc->materials[i].kind <= LUM_MAT_EMISSIVE;
+    // its big spheres (grounds: radius from kBigSphere up, a few at most) stay out of the BVH; every
+    // walk tests them first (walk_warp).  Closest hits do not depend on the order of the tests.
+    std::vector<uint32_t> in_tree, big;
+    for (size_t k = 0; k < F.prims.size(); ++k)
+        (sph && F.prims[k].rec[3] >= lum::kBigSphere ? big : in_tree).push_back((uint32_t)k);
+    if (big.size() > (size_t)lum::kMaxBigSpheres) {
+        in_tree.resize(F.prims.size());
+        for (size_t k = 0; k < in_tree.size(); ++k) in_tree[k] = (uint32_t)k;
+        big.clear();
+    }
+
+    std::vector<lum::BuildBox> boxes(in_tree.size());
+    for (size_t i = 0; i < in_tree.size(); ++i) boxes[i] = F.prims[in_tree[i]].box;
     // relative test costs in the SAH: a quad test reads four 16-byte records against one to
     // three for the others; weighting quads 2 made the box-room frame 6% faster, while sphere
     // and triangle scenes measured best at the plain weight 1
-    std::vector<float> weights(F.prims.size());
-    for (size_t i = 0; i < F.prims.size(); ++i) weights[i] = F.prims[i].type == lum::PT_QUAD ? 2.0f : 1.0f;
+    std::vector<float> weights(in_tree.size());
+    for (size_t i = 0; i < in_tree.size(); ++i) weights[i] = F.prims[in_tree[i]].type == lum::PT_QUAD ? 2.0f : 1.0f;
     lum::BvhOptions opt;
     lum::BvhResult bvh = lum::build_bvh(boxes, opt, &weights);
+    for (uint32_t& k : bvh.order) k = in_tree[k];
+    bvh.order.insert(bvh.order.end(), big.begin(), big.end());
     if (bvh.max_depth > (uint32_t)lum::kMaxBvhDepth)
         return fail(LUM_ERR_TOO_LARGE, "BVH depth %u exceeds the traversal stack", bvh.max_depth);
 
@@ -1087,13 +1107,8 @@ lum_status lum_scene_create(const lum_scene_desc* desc, lum_scene** out) {
     D.n_lights = (int32_t)lights.size();
     D.n_planes = (int32_t)F.planes.size();
     D.n_mats = (int32_t)mats.size();
-    // the sphere-and-basic-materials kernel class (planes are tested in the general way)
-    bool sph = true;
-    for (size_t k = 0; k < np && sph; ++k)   // static spheres: record 1's w (moving flag) is 0
-        sph = (meta[k] & 15) == lum::PT_SPHERE && prims[16 * k + 7] == 0.0f;
-    for (uint32_t i = 0; i < desc->n_materials && sph; ++i)
-        sph = desc->materials[i].kind >= LUM_MAT_LAMBERTIAN && desc->materials[i].kind <= LUM_MAT_EMISSIVE;
     D.spheres_basic = sph ? 1 : 0;
+    D.n_big = (int32_t)big.size();
     // the scene class of the general megakernel build: the primitive types and light kinds
     // present (planes are tested apart from the BVH in every class)
     {

@@ -258,6 +258,7 @@ static int render_occupancy() {
     static const int occ = [] {   // initialised once, thread-safe
         for (auto fn : {k_render<false, false, false, false>, k_render<false, false, true, false>,
                         k_render<false, true, false, false>, k_render<false, true, true, false>,
+                        k_render<false, true, false, false, CLS_GROUND>, k_render<false, true, true, false, CLS_GROUND>,
                         k_render<false, false, false, true>, k_render<false, false, true, true>,
                         k_render<true, false, true, false>, k_render<true, true, true, false>,
                         k_render<false, false, false, false, CLS_QUAD>, k_render<false, false, true, false, CLS_QUAD>,
@@ -393,7 +394,9 @@ static cudaError_t launch_render_t(const SceneDev& S, const RenderDev& R, float*
     const bool nee = COUNT || S.n_lights > 0;
     const bool sph = !COUNT && !R.ext && S.spheres_basic;
     const int cls = (COUNT || R.ext || sph) ? (int)CLS_ALL : S.cls;
-    auto kernel = R.ext ? (nee ? k_render<COUNT, true, true, false> : k_render<COUNT, true, COUNT, false>)
+    auto kernel = R.ext && S.n_big > 0 ? (nee ? k_render<COUNT, true, true, false, CLS_GROUND>
+                                              : k_render<COUNT, true, COUNT, false, CLS_GROUND>)
+                : R.ext ? (nee ? k_render<COUNT, true, true, false> : k_render<COUNT, true, COUNT, false>)
                 : sph   ? (nee ? k_render<COUNT, false, true, !COUNT> : k_render<COUNT, false, COUNT, !COUNT>)
                 : cls == CLS_QUAD ? (nee ? k_render<COUNT, false, true, false, CLS_QUAD>
                                          : k_render<COUNT, false, COUNT, false, CLS_QUAD>)

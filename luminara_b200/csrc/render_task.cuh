@@ -69,7 +69,8 @@ __device__ __forceinline__ void path_step(const SceneDev& S, const RenderDev& R,
     r.o = P.ray.o;
     r.d = shadow ? pend.dir : P.ray.d;
     r.time = shadow ? 0.0f : P.ray.time;                      // Ray::new (render.rs:1457)
-    if (act && !walking) {
+    const bool fresh = act && !walking;
+    if (fresh) {
         h.t = shadow ? (EXT ? fabsf(pend.tmax) : pend.tmax) : CUDART_INF_F;
         h.prim = -1;
         h.b1 = h.b2 = 0.0f;
@@ -78,7 +79,8 @@ __device__ __forceinline__ void path_step(const SceneDev& S, const RenderDev& R,
         found = false;
     }
     constexpr unsigned full = 0xffffffffu;
-    const bool done = walk_warp<COUNT, SPH, SUSPEND, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err, act, tally);
+    const bool done = walk_warp<COUNT, SPH, SUSPEND, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err, act, fresh,
+                                                             tally);
     walking = act && !done;
     __syncwarp(full);   // the lanes shade together
     if (done && shadow) {

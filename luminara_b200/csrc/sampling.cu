@@ -285,6 +285,7 @@ cudaError_t launch_render_sampled(const SceneDev& S, const RenderDev& R, const S
     };
     using Yes = std::true_type;
     using No = std::false_type;
+    if (R.ext && S.n_big > 0) return go(Yes(), No(), std::integral_constant<int, CLS_GROUND>());
     if (R.ext) return go(Yes(), No(), std::integral_constant<int, CLS_ALL>());
     if (S.spheres_basic) return go(No(), Yes(), std::integral_constant<int, CLS_ALL>());
     if (S.cls == CLS_QUAD) return go(No(), No(), std::integral_constant<int, CLS_QUAD>());

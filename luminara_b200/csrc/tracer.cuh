@@ -117,12 +117,13 @@ __device__ __forceinline__ float4 ldp(const SceneDev& S, int i, int k) {
 // Spheres of radius >= kBigSphere (ground spheres) evaluate o - c and |o - c|^2 - r^2 in
 // f64: in f32 that difference loses ~r * 6e-8 absolutely, which near the surface of an
 // r = 1000 sphere is a large relative error of the near root.
-constexpr float kBigSphere = 32.0f;
 // a = |d|^2 and ia = 1 / a are the ray's (the caller may compute them once per ray).
+// BIG: r >= kBigSphere is known.
+template <bool BIG = false>
 __device__ __forceinline__ bool sphere_roots(V c, float r, const Ray& ray, float a, float ia, float& t0, float& t1) {
     V oc;
     float cc;
-    if (r >= kBigSphere) {
+    if (BIG || r >= kBigSphere) {
         double dx = (double)ray.o.x - (double)c.x, dy = (double)ray.o.y - (double)c.y, dz = (double)ray.o.z - (double)c.z;
         oc = mk((float)dx, (float)dy, (float)dz);
         cc = (float)fma(dx, dx, fma(dy, dy, fma(dz, dz, -(double)r * (double)r)));
@@ -149,13 +150,14 @@ __device__ __forceinline__ bool sphere_roots(V c, float r, const Ray& ray, float
 
 // sphere.rs:24-45: near root if in [tmin, tmax], else far root.  ia: 1 / |d|^2 of the ray, or 0
 // to compute it here.
+template <bool BIG = false>
 __device__ __forceinline__ bool hit_sphere(float4 a, float4 b, const Ray& ray, float tmin, float tmax, float& t,
                                            float ia = 0.0f) {
     V c = xyz(a);
     if (b.w != 0.0f) c = fma3(xyz(b) - c, ray.time, c);   // MovingSphere::center_at
     float t0, t1;
     const float aa = len2(ray.d);
-    if (!sphere_roots(c, a.w, ray, aa, ia != 0.0f ? ia : 1.0f / aa, t0, t1)) return false;
+    if (!sphere_roots<BIG>(c, a.w, ray, aa, ia != 0.0f ? ia : 1.0f / aa, t0, t1)) return false;
     if (t0 >= tmin && t0 <= tmax) { t = t0; return true; }
     if (t1 >= tmin && t1 <= tmax) { t = t1; return true; }
     return false;
@@ -275,8 +277,13 @@ static __device__ __noinline__ bool hit_fog_cold(int type, float4 a, float4 b, f
 enum : int {
     CLS_ALL = 0,    // every primitive type and light kind
     CLS_QUAD = 1,   // quads (rects, boxes) with rect lights (box room, quad scenes)
-    CLS_MESH = 2    // triangles, disks and media with disk and rect lights (meshes)
+    CLS_MESH = 2,   // triangles, disks and media with disk and rect lights (meshes)
+    CLS_GROUND = 3  // CLS_ALL, and big spheres apart from the BVH (SceneDev::n_big)
 };
+template <int CLS>
+__host__ __device__ constexpr bool cls_has_big() { return CLS == CLS_GROUND; }
+template <int CLS>
+__host__ __device__ constexpr bool cls_is_all() { return CLS == CLS_ALL || CLS == CLS_GROUND; }
 
 // Unroll factor of the Philox rounds in a scene-class build.  The mesh class's megakernel is
 // bound by instruction fetch (no_instructions is a quarter of its stall samples), and each
@@ -287,12 +294,12 @@ template <int CLS>
 constexpr int philox_unroll() { return CLS == CLS_MESH ? 2 : 10; }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_prim(int type) {
-    return CLS == CLS_ALL || (CLS == CLS_QUAD && type == PT_QUAD) ||
+    return cls_is_all<CLS>() || (CLS == CLS_QUAD && type == PT_QUAD) ||
            (CLS == CLS_MESH && (type == PT_TRIANGLE || type == PT_DISK || type == PT_FOG_SPHERE || type == PT_FOG_BOX));
 }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_light(int kind) {   // 1 sphere, 2 rect, 3 disk
-    return CLS == CLS_ALL || (CLS == CLS_QUAD && kind == 2) || (CLS == CLS_MESH && (kind == 2 || kind == 3));
+    return cls_is_all<CLS>() || (CLS == CLS_QUAD && kind == 2) || (CLS == CLS_MESH && (kind == 2 || kind == 3));
 }
 
 // One primitive test; updates the closest hit when t is within [tmin, hit.t].  The record carries
@@ -488,10 +495,10 @@ struct Trav {
 // mesh and lost 7-9% on the room and the materials' scene; leaving it only when no lane can
 // walk on (no vote on leaves) lost 4-13%; leaving the leaf loop with 2, 6 or 12 lanes' leaves
 // unfinished lost 2-10%; branches instead of predicated stack accesses lost up to 3%.
-template <bool COUNT = false, bool SPH = false, int SUSPEND = 0, int CLS = CLS_ALL>
+template <bool COUNT = false, bool SPH = false, int SUSPEND = 0, int CLS = CLS_GROUND>
 __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, float tmin, bool any, Hit& hit,
                                           bool& found, Trav& tv, int* stack, uint32_t& err, bool act,
-                                          TestTally* tl = nullptr) {
+                                          bool fresh, TestTally* tl = nullptr) {
     constexpr unsigned full = 0xffffffffu;
     // Reciprocals of direction components clamped away from zero: the FMA slab form
     // lo*inv - o*inv would give inf - inf = NaN for an axis-parallel ray, while a finite
@@ -511,6 +518,24 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
     uint32_t sp = base + (uint32_t)tv.sp;      // address of the top entry
     int node = act ? tv.node : kSentinel;      // inner node index, leaf (< 0) or kSentinel
     int leaf = 0;                              // postponed leaf (< 0) or 0
+    // The big spheres, for all new walks of the warp at once: in the tree a ground was a leaf that nearly
+    // every ray visited and tested in f64 a few lanes at a time.  Found first, it also shortens the
+    // ray.  Sphere field (64 spp) 19.9 -> 19.1 ms, adaptive 26.4 -> 25.0, same images; only the builds
+    // that meet such scenes carry it (general scenes 2-10% slower with it).
+    if constexpr (cls_has_big<CLS>() || SPH || COUNT) {
+        for (int k = S.n_prims - S.n_big; k < S.n_prims; ++k) {
+            if constexpr (COUNT) tl->prim[PT_SPHERE] += fresh ? 1 : 0;
+            const float4 c = ldp(S, k, 0);
+            float t;
+            if (fresh && !(any && found) &&
+                hit_sphere<true>(c, make_float4(0.0f, 0.0f, 0.0f, 0.0f), ray, tmin, hit.t, t, ia_ray)) {
+                hit.t = t;
+                hit.prim = k;
+                found = true;
+                if (any) node = kSentinel;
+            }
+        }
+    }
     for (;;) {
         for (;;) {
             if ((unsigned)node < (unsigned)kSentinel) {
@@ -593,7 +618,7 @@ __device__ __forceinline__ bool trace(const SceneDev& S, const Ray& ray, float t
                                       uint32_t& err, bool act, TestTally* tl = nullptr) {
     bool found = false;
     Trav tv{S.n_nodes > 0 ? 0 : kSentinel, 0};
-    walk_warp<COUNT, SPH, 0>(S, ray, tmin, any, hit, found, tv, stack, err, act, tl);
+    walk_warp<COUNT, SPH, 0, CLS_GROUND>(S, ray, tmin, any, hit, found, tv, stack, err, act, act, tl);
     return found;
 }
 

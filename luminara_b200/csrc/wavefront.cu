@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(128, 5) k_render_multi(Tables T, const unsigne
         const uint32_t tw = min(8u, R.w - x0), th = min(4u, R.h - y0);
         const uint32_t s_lo = R.s_begin + group * grp.y;
         const uint32_t s_hi = min(R.s_end, s_lo + grp.y);
-        tile_task<false>(S, R, x0, y0, tw, th, s_lo, s_hi, s_acc[wid], &s_next[wid], s_exit[wid], stack, err, nseg,
+        tile_task<false, true, true, false, LUM_SUSPEND_LANES, CLS_GROUND>(S, R, x0, y0, tw, th, s_lo, s_hi, s_acc[wid], &s_next[wid], s_exit[wid], stack, err, nseg,
                          nsh, nullptr);
         if (lane < (int)(tw * th)) {
             const uint32_t i = x0 + lane % tw, j = y0 + lane / tw;

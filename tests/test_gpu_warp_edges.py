@@ -10,7 +10,7 @@ import pytest
 import luminara_b200 as L
 from luminara_b200 import workloads as W
 
-from .helpers import random_rays, to_gpu_rays
+from .helpers import random_rays, to_gpu_rays, to_orc_rays
 
 pytestmark = pytest.mark.gpu
 
@@ -78,3 +78,39 @@ def test_adaptive_classes_match_the_keyed_oracle(name, size):
     assert st.paths == 25 * size[0] * size[1]
     ref = O.OracleScene(world).render(cfg, mode=O.MODE_KEYED)[0]
     assert (np.abs(img - ref) <= 2e-3 * (1 + np.abs(ref))).all(-1).mean() >= (0.95 if name == "zoo" else 0.97)
+
+
+@pytest.mark.parametrize("n_big,n_small", [(1, 0), (1, 40), (4, 40), (5, 40), (3, 0)])
+def test_big_spheres_beside_the_tree(n_big, n_small):
+    """Spheres of radius 32 and more stay out of a sphere scene's tree, up to four of them: every
+    render mode gives the same image, and closest hits and occlusion are the oracle's."""
+    import oracle as O
+    from luminara_b200 import abi
+    rng = np.random.default_rng(10 * n_big + n_small)
+    w = L.World()
+    for k in range(n_big):
+        r = 32.0 if k == 1 else 100.0 * (k + 1)
+        w.add(L.Sphere((40.0 * k, -r - 0.01 * k, 5.0 * k), r, L.Lambertian((0.3 + 0.1 * k, 0.5, 0.4))))
+    for _ in range(n_small):
+        w.add(L.Sphere(tuple(rng.uniform((-4, 0.2, -4), (4, 1.5, 4))), 0.3, L.Metal((0.8, 0.7, 0.6), 0.2)))
+    w.camera = L.CameraConfig(look_from=(6, 2, 6), look_at=(0, 0.5, 0), aspect_ratio=37 / 21)
+    cfg = L.RenderConfig(width=37, height=21, samples_per_pixel=9, max_depth=6, seed=5)
+    sc = L.GpuScene(w)
+    img, _ = sc.render(cfg)
+    for mode in (abi.BATCH_WAVEFRONT, abi.BATCH_MEGAKERNEL, abi.BATCH_STREAMS):
+        batch = L.Batch([sc], [cfg], config={"mode": mode})
+        np.testing.assert_array_equal(batch.render()[0][0], img)
+        batch.close()
+    orc = O.OracleScene(w)
+    for c in (cfg, L.RenderConfig(**{**cfg.__dict__, "background": abi.BG_STARFIELD, "bg_star_density": 0.2,
+                                     "bg_star_brightness": 1.0})):
+        got, ref = sc.render(c)[0], orc.render(c, mode=O.MODE_KEYED)[0]
+        assert (np.abs(got - ref) <= 2e-3 * (1 + np.abs(ref))).all(-1).mean() >= 0.97
+    o, d, t0, t1 = random_rays(rng, 2000, (-8, 0.05, -8), (8, 6, 8))
+    hits, want = sc.intersect(to_gpu_rays(o, d, t0, t1)), orc.intersect(to_orc_rays(o, d, t0, t1))
+    same = hits["prim_id"] == want["prim_id"]
+    assert same.mean() >= 0.995 and (want["prim_id"] >= 0).any()
+    hit = same & (want["prim_id"] >= 0)
+    np.testing.assert_allclose(hits["t"][hit], want["t"][hit], rtol=2e-3, atol=2e-4)
+    assert ((sc.occluded(to_gpu_rays(o, d, t0, t1)) != 0) == (want["prim_id"] >= 0)).mean() >= 0.995
+    sc.close()
