@@ -23,19 +23,14 @@
 namespace lum {
 
 constexpr int kRenderThreads = 128;
-// Minimum resident blocks per SM requested from the register allocator: 7 (72 registers) for the
-// general build and the scene classes, 8 (64 registers) for the build with the other materials.
-// More warps to hide the dependent node and primitive fetches outweigh the spills (40-130 bytes)
-// up to there.  On B200 with warp-convergent walks: general build (twelve mixed scenes) 5 / 6 / 7 /
-// 8 blocks 186.9 / 177.4 / 171.7 / 181.5 ms; other materials 14.8 / 14.1 / 13.4 / 13.1 ms; classes 6
-// / 7 / 8 blocks: dense mesh 18.1 / 17.5 / 17.5 ms, quads 8.11 / 7.91 / 8.00, box room 1.72 / 1.71 /
-// 1.74.  The sphere builds use 7 blocks without lights (no spills; 6 and 8 blocks the same within
-// 1%) and 6 with them.
+// Minimum resident blocks per SM requested from the register allocator: 7 (72 registers).  More warps
+// to hide the dependent node and primitive fetches outweigh the spills (40-130 bytes) up to there.
+// On B200 with warp-convergent walks and the rare code out of line: general build (twelve mixed
+// scenes) 6 / 7 / 8 blocks 150.2 / 145.4 / 147.8 ms, other materials 7 / 8 / 9 10.8 / 11.0 / 10.9; classes 6
+// / 7 / 8 blocks: dense mesh 17.2 / 16.7 / 16.7 ms, quads 7.70 / 7.60 / 7.69, box room 1.64 / 1.63 /
+// 1.65.  The sphere builds use 7 blocks without lights (6 and 8 the same within 1%) and 6 with them.
 #ifndef LUM_RENDER_MIN_BLOCKS
 #define LUM_RENDER_MIN_BLOCKS 7
-#endif
-#ifndef LUM_RENDER_EXT_BLOCKS
-#define LUM_RENDER_EXT_BLOCKS 8
 #endif
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -68,7 +63,7 @@ __device__ __forceinline__ void flush_counters(WorkCounters* wc, uint32_t err, u
 // CLS (CLS_QUAD, CLS_MESH): general builds carrying only the primitive tests and light samplers
 // of one scene class (SceneDev::cls).
 template <bool COUNT, bool EXT, bool NEE, bool SPH, int CLS = CLS_ALL>
-__global__ void __launch_bounds__(kRenderThreads, SPH ? (NEE ? 6 : 7) : EXT ? LUM_RENDER_EXT_BLOCKS : LUM_RENDER_MIN_BLOCKS)
+__global__ void __launch_bounds__(kRenderThreads, SPH ? (NEE ? 6 : 7) : LUM_RENDER_MIN_BLOCKS)
     k_render(SceneDev S, RenderDev R, float* __restrict__ out, WorkCounters* wc, TaskPlan TP) {
     extern __shared__ int s_stack[];
     __shared__ unsigned long long s_acc[kRenderThreads / 32][32][4];

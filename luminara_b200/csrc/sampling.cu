@@ -82,7 +82,7 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
                 if (centre)
                     start_path_centre(S, R, gi, gj, pixel, P);
                 else
-                    start_path<philox_unroll<CLS>()>(S, R, gi, gj, pixel, st_lo + k, P);
+                    start_path<philox_unroll<CLS, SPH>()>(S, R, gi, gj, pixel, st_lo + k, P);
                 state = R.max_depth > 0 ? ST_CLOSEST : ST_DONE;
             }
         }

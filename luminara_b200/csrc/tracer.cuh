@@ -82,6 +82,17 @@ __device__ __forceinline__ float4 draw4(uint32_t k0, uint32_t k1, uint32_t pixel
     uint4 o = philox<U>(make_uint4(pixel, stratum, bounce, call), k0, k1);
     return make_float4(u24(o.x), u24(o.y), u24(o.z), u24(o.w));
 }
+// The rare draws (dispersion, Blend, Subsurface, moving spheres) out of line, as the other code that few
+// paths or scenes reach: pixel filters but the box, checkers, backgrounds but sky and solid, the
+// panorama camera, media.  Inlined, they made the kernels' loops wait for instructions (2.2 stalled
+// warps per issue on mixed scenes and meshes).  On B200 together, same images: twelve mixed scenes
+// 160 -> 145 ms, the materials' scene 13.0 -> 11.0, dense mesh (16 spp) 17.2 -> 16.7, quads 7.63 -> 7.60.
+// The light sampler, the disk test and the other materials' scatter stay inline: out of line they
+// gained nothing or lost 5-8%.
+static __device__ __noinline__ float4 draw4_cold(uint32_t k0, uint32_t k1, uint32_t pixel, uint32_t stratum, uint32_t bounce,
+                                                 uint32_t call) {
+    return draw4<2>(k0, k1, pixel, stratum, bounce, call);
+}
 enum : uint32_t { CALL_CAMERA = 0, CALL_CAMERA2 = 1, CALL_SCATTER = 2, CALL_NEE = 3, CALL_EXTRA = 4, CALL_BLEND = 5 };
 
 // Direct (rejection-free) samplers; same distributions as src/vec3.rs:96-122.
@@ -261,10 +272,8 @@ __device__ __forceinline__ bool hit_fog(int type, float4 a, float4 b, float4 c, 
     return true;
 }
 
-// hit_fog out of line, for the mesh class's leaf loop (CLS_MESH): that build is bound by
-// instruction fetch, and the fog test (two box or sphere roots and the f64 free-flight hash)
-// runs for a handful of primitives only.  With the light sampler out of line as well the dense
-// mesh ran 173.3 -> 169.8 ms on B200 (fog test alone: 172.1 ms); the other builds inline both.
+// hit_fog out of line (see draw4_cold): two box or sphere roots and the f64 free-flight hash, for a
+// handful of primitives.
 static __device__ __noinline__ bool hit_fog_cold(int type, float4 a, float4 b, float4 c, const Ray& ray, float tmin,
                                                  float tmax, float& t) {
     return hit_fog(type, a, b, c, ray, tmin, tmax, t);
@@ -285,13 +294,13 @@ __host__ __device__ constexpr bool cls_has_big() { return CLS == CLS_GROUND; }
 template <int CLS>
 __host__ __device__ constexpr bool cls_is_all() { return CLS == CLS_ALL || CLS == CLS_GROUND; }
 
-// Unroll factor of the Philox rounds in a scene-class build.  The mesh class's megakernel is
-// bound by instruction fetch (no_instructions is a quarter of its stall samples), and each
-// inlined draw site carries the ten rounds: rolled by two they shrink it, and the dense mesh
-// ran 186.1 -> 173.3 ms on B200; the sphere field, bound by issue, ran 6% slower that way and
-// keeps them unrolled, as do the other classes (box room 1% slower rolled).
-template <int CLS>
-constexpr int philox_unroll() { return CLS == CLS_MESH ? 2 : 10; }
+// Unroll factor of the Philox rounds in a build.  The mesh, general and other-materials builds are bound
+// by instruction fetch, and each inlined draw site carries the ten rounds: rolled by two the mesh
+// ran 186.1 -> 173.3 ms on B200, mixed scenes 150.5 -> 148.8, the materials' scene 11.3 -> 11.2; the
+// sphere field, bound by issue, runs 4-6% slower that way and keeps them unrolled, as does the
+// quad class (box room 1% slower rolled).
+template <int CLS, bool SPH = false>
+constexpr int philox_unroll() { return CLS == CLS_QUAD || SPH ? 10 : 2; }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_prim(int type) {
     return cls_is_all<CLS>() || (CLS == CLS_QUAD && type == PT_QUAD) ||
@@ -359,7 +368,7 @@ __device__ __forceinline__ bool test_prim(const SceneDev& S, int i, const Ray& r
         }
         default: {
             if constexpr (!cls_has_prim<CLS>(PT_FOG_BOX)) return false;
-            const bool fog_hit = CLS == CLS_MESH ? hit_fog_cold(type, a, b, c, ray, tmin, hit.t, t)
+            const bool fog_hit = CLS != CLS_QUAD ? hit_fog_cold(type, a, b, c, ray, tmin, hit.t, t)
                                                  : hit_fog(type, a, b, c, ray, tmin, hit.t, t);
             if (fog_hit) { hit.t = t; hit.prim = i; return true; }
             return false;
@@ -686,12 +695,13 @@ __device__ __forceinline__ Surface surface_of(const SceneDev& S, const Ray& ray,
 }
 
 // ------------------------------------------------------------------------------ shading
-__device__ __forceinline__ V tex_value(const MatDev& m, V p) {           // texture.rs:19-50
-    if (m.tex == 0) return mk(m.color);
+static __device__ __noinline__ V checker_cold(const MatDev* mp, V p) {           // texture.rs:19-50
+    const MatDev& m = *mp;
     float inv = 1.0f / m.tex_scale;
     long long x = (long long)floorf(p.x * inv), y = (long long)floorf(p.y * inv), z = (long long)floorf(p.z * inv);
     return ((x + y + z) % 2 == 0) ? mk(m.color) : mk(m.color2);
 }
+__device__ __forceinline__ V tex_value(const MatDev& m, V p) { return m.tex == 0 ? mk(m.color) : checker_cold(&m, p); }
 
 __device__ __forceinline__ V emitted(const MatDev& m, V p) {           // material.rs:241-243
     return m.kind == 4 ? tex_value(m, p) * m.intensity : mk(0.0f, 0.0f, 0.0f);
@@ -712,13 +722,12 @@ __device__ __forceinline__ V fresnel(float cos_t, V f0) {              // materi
     return f0 * (1.0f - t) + mk(t, t, t);
 }
 
-// material.rs:297-319 with tan(theta) evaluated directly (same angle, no atan/sin/cos).
-__device__ __forceinline__ V ggx_normal(V n, float alpha, float r1, float r2) {
+// material.rs:297-319 with tan(theta) evaluated directly (same angle, no atan/sin/cos); sp, cp: the
+// azimuth's sine and cosine.
+__device__ __forceinline__ V ggx_normal(V n, float alpha, float r1, float sp, float cp) {
     float tan2 = alpha * alpha * r1 / (1.0f - r1 + 1e-10f);
     float ct = rsqrtf(1.0f + tan2);
     float st = sqrtf(tan2) * ct;
-    float sp, cp;
-    sincospif(2.0f * r2, &sp, &cp);
     V up = fabsf(n.y) < 0.999f ? mk(0.f, 1.f, 0.f) : mk(1.f, 0.f, 0.f);
     V tg = unit(cross(up, n));
     V bt = cross(n, tg);
@@ -738,7 +747,7 @@ enum : int { MAT_BLEND = 7 };
 __device__ __forceinline__ const MatDev* blend_walk(const MatDev* mats, const MatDev* m, uint32_t key0,
                                                         uint32_t key1, uint32_t pixel, uint32_t stratum,
                                                         uint32_t bounce) {
-    const float4 u = draw4(key0, key1, pixel, stratum, bounce, CALL_BLEND);
+    const float4 u = draw4_cold(key0, key1, pixel, stratum, bounce, CALL_BLEND);
     const float uu[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int l = 0; l < kMaxBlendDepth; ++l) {
@@ -782,7 +791,8 @@ struct ScatterMore {
     V dir, att, org;
     bool ok;
 };
-__device__ __forceinline__ ScatterMore scatter_more(const MatDev* mp, V rd, V hp, V hn, float4 s, uint32_t key0,
+__device__ __forceinline__ ScatterMore scatter_more(
+const MatDev* mp, V rd, V hp, V hn, float4 s, uint32_t key0,
                                                        uint32_t key1, uint32_t pixel, uint32_t stratum,
                                                        uint32_t bounce) {
     const MatDev& m = *mp;
@@ -900,7 +910,7 @@ __device__ __forceinline__ ScatterMore scatter_more(const MatDev* mp, V rd, V hp
             const float mfp = m.extra[0];
             float step = -mfp * logf(fmaxf(s.y, 1e-10f));
             out.org = sf.p + unit_vector(s.z, s.w) * step;
-            float4 ex = draw4(key0, key1, pixel, stratum, bounce, CALL_EXTRA);
+            float4 ex = draw4_cold(key0, key1, pixel, stratum, bounce, CALL_EXTRA);
             V d = sf.n + unit_vector(ex.x, ex.y);
             out.dir = near_zero(d) ? sf.n : unit(d);
             const float k = -step / mfp;
@@ -926,9 +936,23 @@ __device__ __forceinline__ bool scatter(const MatDev& m, const Ray& ray, const S
     if constexpr (SPH) {
         if (KIND < 0 && m.kind > 3) return false;                      // Emissive: no scatter
     }
-    switch (KIND >= 0 ? KIND : m.kind) {
+    // The materials' random unit vector, evaluated once for all lanes of the warp (Lambertian, Metal and
+    // Isotropic draw it from s.x, s.y; rough Dielectric and both Microfacet lobes' azimuths from s.y,
+    // s.z): each material inlined its own copy, for its own lanes, in kernels bound by instruction
+    // fetch and divergence.  Twelve mixed scenes 169 -> 159 ms, dense mesh (16 spp) 17.6 -> 17.2,
+    // quads 7.76 -> 7.62, box room 1.66 -> 1.65, sphere field (64 spp) 18.9 -> 18.8.
+    const int kind = KIND >= 0 ? KIND : m.kind;
+    const bool late = kind == 3 || kind == 5;
+    float us, uc;
+    sincospif(2.0f * (late ? s.z : s.y), &us, &uc);
+    const float uz = 1.0f - 2.0f * (late ? s.y : s.x);
+    const float ur = sqrtf(fmaxf(0.0f, 1.0f - uz * uz));
+    // n plus the unit vector, fused explicitly (see add_light), and the unit vector times x
+    auto about = [&](V n) { return V{fmaf(ur, uc, n.x), fmaf(ur, us, n.y), n.z + uz}; };
+    auto times = [&](float x) { return V{ur * uc, ur * us, uz} * x; };
+    switch (kind) {
         case 1: {                                                      // material.rs:59-71
-            V d = sf.n + unit_vector(s.x, s.y);
+            V d = about(sf.n);
             if (near_zero(d)) d = sf.n;
             out.dir = d;
             out.att = tex_value(m, sf.p);
@@ -936,7 +960,7 @@ __device__ __forceinline__ bool scatter(const MatDev& m, const Ray& ray, const S
         }
         case 2: {                                                      // material.rs:94-106
             V refl = reflect(unit(ray.d), sf.n);
-            V sc = refl + in_unit_sphere(s.x, s.y, s.z) * m.fuzz;
+            V sc = refl + times(cbrtf(s.z)) * m.fuzz;
             if (dot(sc, sf.n) > 0.0f) {
                 out.dir = sc;
                 out.att = mk(m.color);
@@ -948,7 +972,7 @@ __device__ __forceinline__ bool scatter(const MatDev& m, const Ray& ray, const S
             float ior = m.ior;
             V chan = mk(1.f, 1.f, 1.f);
             if (m.dispersion > 0.0f) {
-                float4 ex = draw4<U>(R.key0, R.key1, pixel, stratum, bounce, CALL_EXTRA);
+                float4 ex = draw4_cold(R.key0, R.key1, pixel, stratum, bounce, CALL_EXTRA);
                 uint32_t ch = (uint32_t)(ex.x * 3.0f);
                 ior += ch == 0 ? -m.dispersion : (ch == 1 ? 0.0f : m.dispersion);
                 chan = ch == 0 ? mk(3.f, 0.f, 0.f) : (ch == 1 ? mk(0.f, 3.f, 0.f) : mk(0.f, 0.f, 3.f));
@@ -964,7 +988,7 @@ __device__ __forceinline__ bool scatter(const MatDev& m, const Ray& ray, const S
                 V rp = (ud + sf.n * ct) * eta;
                 d = rp + sf.n * -sqrtf(fabsf(1.0f - len2(rp)));
             }
-            if (m.roughness > 0.0f) d = d + in_unit_sphere(s.y, s.z, s.w) * m.roughness;
+            if (m.roughness > 0.0f) d = d + times(cbrtf(s.w)) * m.roughness;
             V att;
             if (!sf.front && !m.tint_white)
                 att = mk(__expf(-(1.0f - m.tint[0]) * hit_t), __expf(-(1.0f - m.tint[1]) * hit_t),
@@ -986,7 +1010,7 @@ __device__ __forceinline__ bool scatter(const MatDev& m, const Ray& ray, const S
             V fw = fresnel(ndv, f0);
             float sp = fminf(fmaxf((fw.x + fw.y + fw.z) * (1.0f / 3.0f), 0.1f), 0.9f);
             if (s.x < sp) {
-                V h = ggx_normal(n, alpha, s.y, s.z);
+                V h = ggx_normal(n, alpha, s.y, us, uc);
                 V l = h * (2.0f * dot(v, h)) - v;
                 float ndl = dot(n, l);
                 if (ndl <= 0.0f) return false;
@@ -1000,7 +1024,7 @@ __device__ __forceinline__ bool scatter(const MatDev& m, const Ray& ray, const S
                 out.att = w * (1.0f / sp);
                 return true;
             }
-            V d = n + unit_vector(s.y, s.z);
+            V d = about(n);
             if (near_zero(d)) d = n;
             V kd = (mk(1.f, 1.f, 1.f) - fw) * (1.0f - m.metallic);
             out.dir = d;
@@ -1008,7 +1032,7 @@ __device__ __forceinline__ bool scatter(const MatDev& m, const Ray& ray, const S
             return true;
         }
         case 6: {                                                      // constant_medium.rs:81-89
-            out.dir = in_unit_sphere(s.x, s.y, s.z);
+            out.dir = times(cbrtf(s.z));
             out.att = mk(m.color);
             return true;
         }
@@ -1162,10 +1186,9 @@ __device__ __forceinline__ V envmap(const float* env, uint32_t env_w, uint32_t e
 // The unit direction and the gradients' blend are rounded explicitly (see add_light): an image must
 // not depend on which kernel's contraction of y * rsqrt + 1 or a * (1 - t) + b * t it got.
 template <bool EXT = true>
-__device__ __forceinline__ V background(const SceneDev& S, const RenderDev& R, const Ray& r) {  // render.rs:73-171
-    if (R.background == 1) return mk(R.bg_color);
-    const float rl = rsqrtf(len2(r.d));
-    const V ud = V{__fmul_rn(r.d.x, rl), __fmul_rn(r.d.y, rl), __fmul_rn(r.d.z, rl)};
+__device__ __noinline__ V background_cold(const float* env, uint32_t env_w, uint32_t env_h, const RenderDev& R, V rd) {  // render.rs:73-171
+    const float rl = rsqrtf(len2(rd));
+    const V ud = V{__fmul_rn(rd.x, rl), __fmul_rn(rd.y, rl), __fmul_rn(rd.z, rl)};
     const float t = 0.5f * __fadd_rn(ud.y, 1.0f), u = __fsub_rn(1.0f, t);
     auto blend = [t, u](V a, V b) {
         return V{fmaf(b.x, t, __fmul_rn(a.x, u)), fmaf(b.y, t, __fmul_rn(a.y, u)), fmaf(b.z, t, __fmul_rn(a.z, u))};
@@ -1183,9 +1206,17 @@ __device__ __forceinline__ V background(const SceneDev& S, const RenderDev& R, c
     }
     if constexpr (EXT) {
         if (R.background == 4) return starfield(R.star_density, R.star_brightness, ud, t);
-        if (R.background == 5) return envmap(S.env, S.env_w, S.env_h, R.bg_intensity, ud);
+        if (R.background == 5) return envmap(env, env_w, env_h, R.bg_intensity, ud);
     }
     return blend(mk(1.f, 1.f, 1.f), mk(0.5f, 0.7f, 1.0f));
+}
+template <bool EXT = true>
+__device__ __forceinline__ V background(const SceneDev& S, const RenderDev& R, const Ray& r) {  // render.rs:73-171
+    if (R.background == 1) return mk(R.bg_color);
+    if (R.background != 0) return background_cold<EXT>(S.env, S.env_w, S.env_h, R, r.d);
+    const float rl = rsqrtf(len2(r.d));
+    const float t = 0.5f * __fadd_rn(__fmul_rn(r.d.y, rl), 1.0f), u = __fsub_rn(1.0f, t);
+    return V{fmaf(0.5f, t, u), fmaf(0.7f, t, u), fmaf(1.0f, t, u)};
 }
 
 // The pixel filter is written with explicitly rounded operations (no FMA contraction): the
@@ -1205,13 +1236,16 @@ __device__ __forceinline__ float mitchell_1d(float x) {                // render
                                    8.f * b + 24.f * c), 6.f);
     return 0.0f;
 }
-__device__ __forceinline__ float filter_weight(int f, float dx, float dy) {  // render.rs:201-216
+static __device__ __noinline__ float filter_weight_cold(int f, float dx, float dy) {  // render.rs:201-216
     if (f == 1)
         return __fmul_rn(fmaxf(__fsub_rn(1.0f, __fmul_rn(fabsf(dx), 2.0f)), 0.0f),
                          fmaxf(__fsub_rn(1.0f, __fmul_rn(fabsf(dy), 2.0f)), 0.0f));
     if (f == 2) return __expf(__fdiv_rn(-__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), 2.0f * 0.35f * 0.35f));
     if (f == 3) return __fmul_rn(mitchell_1d(__fmul_rn(dx, 2.0f)), mitchell_1d(__fmul_rn(dy, 2.0f)));
     return 1.0f;
+}
+__device__ __forceinline__ float filter_weight(int f, float dx, float dy) {
+    return f == 0 ? 1.0f : filter_weight_cold(f, dx, dy);
 }
 
 // A finished path's contribution to its pixel (render.rs:1692-1701): radiance clamped to
@@ -1251,6 +1285,21 @@ __device__ __forceinline__ float div_by(float a, float b, float r) {
     return fmaf(fmaf(-q, b, a), r, q);
 }
 
+// Direction of the equirectangular camera at (uc, vc); out of line, see draw4_cold.
+static __device__ __noinline__ V panorama_dir(V fwd, V u, V v, float uc, float vc) {
+    // equirectangular (camera.rs:83-90): latitude theta = pi (1 - t), longitude
+    // phi = 2 pi s - pi, unit direction; no lens
+    // (explicitly rounded: the compiler contracts a * b + c into an FMA per call site, and
+    // every kernel must produce the same direction bit for bit)
+    float st_, ct_, sp_, cp_;
+    sincospif(1.0f - vc, &st_, &ct_);
+    sincospif(fmaf(2.0f, uc, -1.0f), &sp_, &cp_);
+    const float a_ = __fmul_rn(st_, cp_), b_ = __fmul_rn(st_, sp_);
+    return mk(fmaf(fwd.x, a_, fmaf(u.x, b_, __fmul_rn(v.x, ct_))),
+                   fmaf(fwd.y, a_, fmaf(u.y, b_, __fmul_rn(v.y, ct_))),
+                   fmaf(fwd.z, a_, fmaf(u.z, b_, __fmul_rn(v.z, ct_))));
+}
+
 // Camera ray through sub-pixel position (jx, jy) of pixel (gi, gj) for stratum st; c holds
 // the stratum's camera draws (z, w: lens) (render.rs:1683-1690, camera.rs:82-102).
 template <int U = 10>
@@ -1263,17 +1312,7 @@ __device__ __forceinline__ void start_path_at(const SceneDev& S, const RenderDev
     const float vc = div_by(y + P.jy, (float)(R.full_h - 1), R.inv_h1);
     const CameraDev& C = S.cam;
     if (C.panorama) {
-        // equirectangular (camera.rs:83-90): latitude theta = pi (1 - t), longitude
-        // phi = 2 pi s - pi, unit direction; no lens
-        // (explicitly rounded: the compiler contracts a * b + c into an FMA per call site, and
-        // every kernel must produce the same direction bit for bit)
-        float st_, ct_, sp_, cp_;
-        sincospif(1.0f - vc, &st_, &ct_);
-        sincospif(fmaf(2.0f, uc, -1.0f), &sp_, &cp_);
-        const float a_ = __fmul_rn(st_, cp_), b_ = __fmul_rn(st_, sp_);
-        const V d = mk(fmaf(C.fwd[0], a_, fmaf(C.u[0], b_, __fmul_rn(C.v[0], ct_))),
-                       fmaf(C.fwd[1], a_, fmaf(C.u[1], b_, __fmul_rn(C.v[1], ct_))),
-                       fmaf(C.fwd[2], a_, fmaf(C.u[2], b_, __fmul_rn(C.v[2], ct_))));
+        const V d = panorama_dir(mk(C.fwd), mk(C.u), mk(C.v), uc, vc);
         P.ray.o = mk(C.origin);
         P.ray.d = d * rsqrtf(len2(d));
     } else {
@@ -1288,7 +1327,7 @@ __device__ __forceinline__ void start_path_at(const SceneDev& S, const RenderDev
     }
     // time matters only to moving spheres; a static scene skips the draw (the keyed draws of
     // the other calls do not depend on it)
-    P.ray.time = S.moving ? draw4<U>(R.key0, R.key1, pixel, st, 0, CALL_CAMERA2).x : 0.0f;
+    P.ray.time = S.moving ? draw4_cold(R.key0, R.key1, pixel, st, 0, CALL_CAMERA2).x : 0.0f;
     P.beta = mk(1.f, 1.f, 1.f);
     P.L = mk(0.f, 0.f, 0.f);
     P.stratum = st;
@@ -1373,11 +1412,11 @@ __device__ __forceinline__ int shade(const SceneDev& S, const RenderDev& R, uint
     const MatDev& m = S.mats[sf.mat];
     V e = P.skip_emission ? mk(0.f, 0.f, 0.f)
                           : (EXT && KIND < 0 ? emitted_at(S, sf.mat, m, sf.p) : emitted(m, sf.p));
-    float4 su = draw4<philox_unroll<CLS>()>(R.key0, R.key1, pixel, P.stratum, P.bounce, CALL_SCATTER);
+    float4 su = draw4<philox_unroll<CLS, SPH>()>(R.key0, R.key1, pixel, P.stratum, P.bounce, CALL_SCATTER);
     Scatter sc;
     sc.org = sf.p;
     const MatDev& ms = EXT && KIND < 0 ? blend_leaf(S, m, R, pixel, P.stratum, P.bounce) : m;
-    if (!scatter<KIND, EXT, SPH, philox_unroll<CLS>()>(ms, P.ray, sf, h.t, su, R, pixel, P.stratum, P.bounce, sc)) {
+    if (!scatter<KIND, EXT, SPH, philox_unroll<CLS, SPH>()>(ms, P.ray, sf, h.t, su, R, pixel, P.stratum, P.bounce, sc)) {
         add_light(P, e);
         return ST_DONE;
     }
@@ -1392,7 +1431,7 @@ __device__ __forceinline__ int shade(const SceneDev& S, const RenderDev& R, uint
     // that ends below no longer reads its ray)
     P.ray.o = sc.org;
     P.ray.d = sc.dir;
-    float4 nu = draw4<philox_unroll<CLS>()>(R.key0, R.key1, pixel, P.stratum, P.bounce, CALL_NEE);
+    float4 nu = draw4<philox_unroll<CLS, SPH>()>(R.key0, R.key1, pixel, P.stratum, P.bounce, CALL_NEE);
     float surv = fminf(fmaxf(fmaxf(fmaxf(sc.att.x, sc.att.y), sc.att.z), 0.05f), 1.0f);
     if (depth < 47 && nu.x > surv) {                                   // Russian roulette
         add_light(P, e);
