@@ -17,7 +17,7 @@
 
 namespace lum {
 
-// Primitive types (low 4 bits of meta, and as an integer in c.w, which no type uses otherwise)
+// Primitive types (low 4 bits of meta, which c.w repeats: no type uses it otherwise)
 enum PrimType : int32_t {
     PT_SPHERE = 0,    // a=(c, r)        b=(c1, moving?1:0)
     PT_QUAD = 1,      // a=(Q, w.Q)      b=(u, |u x v|)    c=(v, -)  d=(w, outward sign); w = (u x v)/|u x v|^2

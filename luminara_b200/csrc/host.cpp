@@ -1013,9 +1013,8 @@ lum_status lum_scene_create(const lum_scene_desc* desc, lum_scene** out) {
     for (size_t k = 0; k < np; ++k) {
         const PrimH& p = F.prims[bvh.order[k]];
         std::memcpy(&prims[16 * k], p.rec, sizeof p.rec);
-        const int32_t type = p.type;                 // record 2's w: the hit tests' type (device_scene.h)
-        std::memcpy(&prims[16 * k + 11], &type, sizeof type);
         meta[k] = (p.material << 4) | p.type;
+        std::memcpy(&prims[16 * k + 11], &meta[k], sizeof meta[k]);   // and in record 2's w (device_scene.h)
         orig[k] = p.orig;
     }
     std::vector<lum::MatDev> mats(desc->n_materials);

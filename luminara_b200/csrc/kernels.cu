@@ -257,7 +257,10 @@ static int render_occupancy() {
                         k_render<false, false, false, true>, k_render<false, false, true, true>,
                         k_render<true, false, true, false>, k_render<true, true, true, false>,
                         k_render<false, false, false, false, CLS_QUAD>, k_render<false, false, true, false, CLS_QUAD>,
-                        k_render<false, false, false, false, CLS_MESH>, k_render<false, false, true, false, CLS_MESH>})
+                        k_render<false, false, false, false, CLS_MESH>, k_render<false, false, true, false, CLS_MESH>,
+                        k_render<false, false, false, false, CLS_MESH_MANY>,
+                        k_render<false, false, true, false, CLS_MESH_MANY>,
+                        k_render<false, false, false, false, CLS_MANY>, k_render<false, false, true, false, CLS_MANY>})
             cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stack_bytes(kRenderThreads));
         int o = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_render<false, false, true, false>, kRenderThreads,
@@ -389,15 +392,20 @@ static cudaError_t launch_render_t(const SceneDev& S, const RenderDev& R, float*
     const bool nee = COUNT || S.n_lights > 0;
     const bool sph = !COUNT && !R.ext && S.spheres_basic;
     const int cls = (COUNT || R.ext || sph) ? (int)CLS_ALL : S.cls;
+    const bool many = !COUNT && S.n_prims >= (cls == CLS_MESH ? kManyTriangles : kManyPrims);
     auto kernel = R.ext && S.n_big > 0 ? (nee ? k_render<COUNT, true, true, false, CLS_GROUND>
                                               : k_render<COUNT, true, COUNT, false, CLS_GROUND>)
                 : R.ext ? (nee ? k_render<COUNT, true, true, false> : k_render<COUNT, true, COUNT, false>)
                 : sph   ? (nee ? k_render<COUNT, false, true, !COUNT> : k_render<COUNT, false, COUNT, !COUNT>)
                 : cls == CLS_QUAD ? (nee ? k_render<COUNT, false, true, false, CLS_QUAD>
                                          : k_render<COUNT, false, COUNT, false, CLS_QUAD>)
+                : cls == CLS_MESH && many ? (nee ? k_render<COUNT, false, true, false, CLS_MESH_MANY>
+                                                 : k_render<COUNT, false, COUNT, false, CLS_MESH_MANY>)
                 : cls == CLS_MESH ? (nee ? k_render<COUNT, false, true, false, CLS_MESH>
                                          : k_render<COUNT, false, COUNT, false, CLS_MESH>)
-                        : (nee ? k_render<COUNT, false, true, false> : k_render<COUNT, false, COUNT, false>);
+                : many ? (nee ? k_render<COUNT, false, true, false, CLS_MANY>
+                              : k_render<COUNT, false, COUNT, false, CLS_MANY>)
+                       : (nee ? k_render<COUNT, false, true, false> : k_render<COUNT, false, COUNT, false>);
     // the traversal stack sized to the scene's BVH; resident blocks for that size
     const size_t smem = stack_smem(S.stack_depth, kRenderThreads);
     if (blocks_per_sm == occ) blocks_per_sm = kernel_occupancy((const void*)kernel, smem);

@@ -287,12 +287,24 @@ enum : int {
     CLS_ALL = 0,    // every primitive type and light kind
     CLS_QUAD = 1,   // quads (rects, boxes) with rect lights (box room, quad scenes)
     CLS_MESH = 2,   // triangles, disks and media with disk and rect lights (meshes)
-    CLS_GROUND = 3  // CLS_ALL, and big spheres apart from the BVH (SceneDev::n_big)
+    CLS_GROUND = 3, // CLS_ALL, and big spheres apart from the BVH (SceneDev::n_big)
+    CLS_MANY = 4,   // CLS_ALL and CLS_MESH for large scenes (kManyPrims, kManyTriangles): their warps turn to
+    CLS_MESH_MANY = 5   // the leaves once at most two lanes still look for one (walk_warp)
 };
+// From these sizes a walk is long enough that the last lanes' search for a leaf costs the others more
+// than turning to the leaves early does.  No lane against two, 64 spp: mesh of 20k triangles 6.40 /
+// 6.50 ms, 82k 6.94 / 6.95, 328k 7.49 / 7.33, 1.3 M (1080p, 16 spp) 16.7 / 16.1; general scenes of 3k
+// 15.7 / 15.8, 10k 20.6 / 20.5, 30k 24.5 / 23.9; 30 to 300 primitives lose 2-4%.  One lane or three gave
+// less at the large end.
+constexpr int kManyPrims = 16384, kManyTriangles = 65536;
+template <int CLS>
+__host__ __device__ constexpr int cls_slack() { return CLS == CLS_MANY || CLS == CLS_MESH_MANY ? 2 : 0; }
+template <int CLS>
+__host__ __device__ constexpr bool cls_is_mesh() { return CLS == CLS_MESH || CLS == CLS_MESH_MANY; }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_big() { return CLS == CLS_GROUND; }
 template <int CLS>
-__host__ __device__ constexpr bool cls_is_all() { return CLS == CLS_ALL || CLS == CLS_GROUND; }
+__host__ __device__ constexpr bool cls_is_all() { return CLS == CLS_ALL || CLS == CLS_GROUND || CLS == CLS_MANY; }
 
 // Unroll factor of the Philox rounds in a build.  The mesh, general and other-materials builds are bound
 // by instruction fetch, and each inlined draw site carries the ten rounds: rolled by two the mesh
@@ -304,11 +316,11 @@ constexpr int philox_unroll() { return CLS == CLS_QUAD || SPH ? 10 : 2; }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_prim(int type) {
     return cls_is_all<CLS>() || (CLS == CLS_QUAD && type == PT_QUAD) ||
-           (CLS == CLS_MESH && (type == PT_TRIANGLE || type == PT_DISK || type == PT_FOG_SPHERE || type == PT_FOG_BOX));
+           (cls_is_mesh<CLS>() && (type == PT_TRIANGLE || type == PT_DISK || type == PT_FOG_SPHERE || type == PT_FOG_BOX));
 }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_light(int kind) {   // 1 sphere, 2 rect, 3 disk
-    return cls_is_all<CLS>() || (CLS == CLS_QUAD && kind == 2) || (CLS == CLS_MESH && (kind == 2 || kind == 3));
+    return cls_is_all<CLS>() || (CLS == CLS_QUAD && kind == 2) || (cls_is_mesh<CLS>() && (kind == 2 || kind == 3));
 }
 
 // One primitive test; updates the closest hit when t is within [tmin, hit.t].  The record carries
@@ -338,7 +350,7 @@ __device__ __forceinline__ bool test_prim(const SceneDev& S, int i, const Ray& r
         return false;
     }
     const float4 b = ldp(S, i, 1), c = ldp(S, i, 2);
-    const int type = __float_as_int(c.w);
+    const int type = __float_as_int(c.w) & 15;
     if constexpr (COUNT) tl->prim[type]++;
     switch (type) {
         case PT_SPHERE: {
@@ -562,7 +574,14 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
                 visit_children(en0, ex0, en1, ex1, link.x, link.y, node, leaf, sp, limit, stride, err);
             }
             // on while some lane that can walk has no leaf yet
-            if (!__any_sync(full, (unsigned)node < (unsigned)kSentinel && leaf == 0)) break;
+            // (builds for large scenes: while more than kSlack such lanes are left)
+            const bool on = (unsigned)node < (unsigned)kSentinel && leaf == 0;
+            constexpr int kSlack = cls_slack<CLS>();
+            if constexpr (kSlack > 0) {
+                if (__popc(__ballot_sync(full, on)) <= kSlack) break;
+            } else {
+                if (!__any_sync(full, on)) break;
+            }
         }
         int k = 0, last = -1;                  // primitives of the leaf to test
         if (leaf < 0) {
@@ -649,7 +668,9 @@ __device__ __forceinline__ Surface surface_of(const SceneDev& S, const Ray& ray,
         on = mk(P.n);
         s.mat = P.material;
     } else {
-        int meta = __ldg(S.meta + h.prim);
+        // material and type: record 2's w, in the L1 since the hit (the sphere class's tests read only
+        // record 0)
+        const int meta = SPH ? __ldg(S.meta + h.prim) : __float_as_int(ldp(S, h.prim, 2).w);
         int type = SPH ? (int)PT_SPHERE : meta & 15;
         s.mat = meta >> 4;
         float4 a = ldp(S, h.prim, 0);
@@ -1446,7 +1467,7 @@ __device__ __forceinline__ int shade(const SceneDev& S, const RenderDev& R, uint
     if (use_nee) {
         Ray sr;
         V contrib;
-        const bool lit = CLS == CLS_MESH ? sample_light_cold<CLS>(S, sf.p, sf.n, sc.att, nu, sr, pend.tmax, contrib)
+        const bool lit = cls_is_mesh<CLS>() ? sample_light_cold<CLS>(S, sf.p, sf.n, sc.att, nu, sr, pend.tmax, contrib)
                                          : sample_light<CLS>(S, sf.p, sf.n, sc.att, nu, sr, pend.tmax, contrib);
         if (lit) {
             pend.dir = sr.d;

@@ -114,3 +114,22 @@ def test_big_spheres_beside_the_tree(n_big, n_small):
     np.testing.assert_allclose(hits["t"][hit], want["t"][hit], rtol=2e-3, atol=2e-4)
     assert ((sc.occluded(to_gpu_rays(o, d, t0, t1)) != 0) == (want["prim_id"] >= 0)).mean() >= 0.995
     sc.close()
+
+
+@pytest.mark.parametrize("kind,n", [("general", 16000), ("general", 17000), ("mesh", 6)])
+def test_large_scene_builds_equal_the_other_modes(kind, n):
+    """Scenes on both sides of the sizes from which warps turn to their leaves early: the same image in
+    every render mode (the batch's kernels never do), and again."""
+    from luminara_b200 import abi
+    if kind == "mesh":
+        world, cfg = W.dense_mesh(61, 35, 4, level=n)                      # 81,920 triangles
+    else:
+        world, cfg = W.uneven_scene(np.random.default_rng(n), n, 61, 35, 4)
+    sc = L.GpuScene(world)
+    img, _ = sc.render(cfg)
+    for mode in (abi.BATCH_WAVEFRONT, abi.BATCH_MEGAKERNEL, abi.BATCH_STREAMS):
+        batch = L.Batch([sc], [cfg], config={"mode": mode})
+        np.testing.assert_array_equal(batch.render()[0][0], img)
+        batch.close()
+    np.testing.assert_array_equal(sc.render(cfg)[0], img)
+    sc.close()
