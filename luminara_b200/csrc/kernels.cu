@@ -293,10 +293,14 @@ static int kernel_occupancy(const void* fn, size_t smem) {
 //   512x512 x 64 spp quads (8192 tiles)     2 groups of 32 strata 10.26 ms, 4 of 16  9.66 ms
 //   256x256 x 64 spp box room (2048 tiles)  7 groups of 10        1.99 ms, 14 of 5   2.02 ms,
 //                                           8 of 8                 1.94 ms
-// and since walks are warp-convergent, groups of at least 4 -> 2 strata (16 spp):
-//   128x128 quads (512 tiles) 0.504 -> 0.410 ms, 320x180 mesh (1800 tiles) 1.16 -> 0.97, 320x180
-//   spheres 0.312 -> 0.297, 128x128 box room 0.297 -> 0.292 (single strata: 0.331);
-// 16 tasks per warp, or groups of 4 strata preferred, lost 2-5% on the larger of these frames.
+// A launch that such groups leave with less than 1.5 tasks per resident warp takes groups of at least 2
+// strata, and one still below 0.5 single strata; at 16 spp, groups of at least 4 / 2 / 1 strata:
+//   64x48 quads 0.330 / 0.236 / 0.208 ms, box room 0.177 / 0.134 / 0.117  (0.1 / 0.2 / 0.4 tasks a warp)
+//   128x128 quads 0.484 / 0.371, spheres 0.198 / 0.146, mesh 0.585 / 0.486        (0.5 / 1.0)
+//   256x144 quads 0.510 / 0.407, box room 0.323 / 0.267                            (1.1 / 2.2)
+//   320x180 quads 0.637 / 0.550, box room 0.336 / 0.363, mesh 0.870 / 0.886        (1.7 / 3.5)
+//   400x225 quads 0.715 / 0.716, box room 0.463 / 0.519, mesh 1.148 / 1.226        (2.7 / 5.5)
+// 16 tasks per warp, or groups of 4 strata preferred, lost 2-5% on larger frames.
 // A larger frame can also split its last LUM_TAIL_TILES_PER_WARP x (resident warps) tiles into
 // LUM_TAIL_GROUPS groups, so that the launch ends on short tasks; on the 1080p frames (spheres
 // 256 spp, dense mesh 144 spp) that gained nothing -- the warps still running at the end of a
@@ -308,7 +312,7 @@ static int kernel_occupancy(const void* fn, size_t smem) {
 #define LUM_SMALL_FRAME_TASKS 8
 #endif
 #ifndef LUM_MIN_GROUP_STRATA
-#define LUM_MIN_GROUP_STRATA 2
+#define LUM_MIN_GROUP_STRATA 4
 #endif
 #ifndef LUM_PREF_GROUP_STRATA
 #define LUM_PREF_GROUP_STRATA 8
@@ -331,7 +335,11 @@ RenderGroups render_groups(const RenderDev& R) {
     uint64_t groups, split;
     if ((uint64_t)R.n_tasks < (uint64_t)LUM_SMALL_FRAME_TILES * warps) {
         groups = ((uint64_t)LUM_SMALL_FRAME_TASKS * warps + R.n_tasks - 1) / R.n_tasks;
-        groups = std::min<uint64_t>(groups, n_st / LUM_MIN_GROUP_STRATA);
+        const uint64_t n = R.n_tasks;
+        uint64_t least = LUM_MIN_GROUP_STRATA;
+        if (2 * n * (n_st / least) < 3 * warps) least = LUM_MIN_GROUP_STRATA / 2;
+        if (2 * n * (n_st / least) < warps) least = 1;
+        groups = std::min<uint64_t>(groups, std::max<uint64_t>(1, n_st / least));
         const uint64_t wide = n_st / LUM_PREF_GROUP_STRATA;   // groups of the preferred size
         if (groups > wide && wide * R.n_tasks >= (uint64_t)LUM_SMALL_FRAME_TILES * warps) groups = wide;
         split = R.n_tasks;

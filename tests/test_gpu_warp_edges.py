@@ -133,3 +133,25 @@ def test_large_scene_builds_equal_the_other_modes(kind, n):
         batch.close()
     np.testing.assert_array_equal(sc.render(cfg)[0], img)
     sc.close()
+
+
+@pytest.mark.parametrize("size", [(64, 48), (128, 128), (320, 180), (640, 360)])
+def test_task_plans_add_up_to_the_same_frame(size):
+    """Frames whose plans split strata into groups of 1, 2, 4 and more: two stratum ranges, each with its
+    own plan, add up to the whole frame's raw sums."""
+    import torch
+    world, cfg = W.box_room(*size, 16, max_depth=3)
+    sc = L.GpuScene(world)
+    def sums(begin, count):
+        cfg.sample_begin, cfg.sample_count = begin, count
+        t = torch.empty((size[1], size[0], 4), dtype=torch.int64, device="cuda")
+        sc.render_sums_device(cfg, t.data_ptr())
+        return t
+    whole, parts = sums(0, 16), sums(0, 5) + sums(5, 11)
+    assert torch.equal(whole, parts)
+    cfg.sample_begin = cfg.sample_count = 0
+    px = torch.empty((size[1], size[0], 3), device="cuda")
+    L.sums_finalize_device(whole.data_ptr(), *size, 1.0, px.data_ptr())
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(px.cpu().numpy(), sc.render(cfg)[0])
+    sc.close()
