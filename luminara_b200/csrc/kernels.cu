@@ -258,6 +258,8 @@ static int render_occupancy() {
                         k_render<true, false, true, false>, k_render<true, true, true, false>,
                         k_render<false, false, false, false, CLS_QUAD>, k_render<false, false, true, false, CLS_QUAD>,
                         k_render<false, false, false, false, CLS_MESH>, k_render<false, false, true, false, CLS_MESH>,
+                        k_render<false, false, false, false, CLS_QUAD_MANY>,
+                        k_render<false, false, true, false, CLS_QUAD_MANY>,
                         k_render<false, false, false, false, CLS_MESH_MANY>,
                         k_render<false, false, true, false, CLS_MESH_MANY>,
                         k_render<false, false, false, false, CLS_MANY>, k_render<false, false, true, false, CLS_MANY>})
@@ -293,7 +295,7 @@ static int kernel_occupancy(const void* fn, size_t smem) {
 //   512x512 x 64 spp quads (8192 tiles)     2 groups of 32 strata 10.26 ms, 4 of 16  9.66 ms
 //   256x256 x 64 spp box room (2048 tiles)  7 groups of 10        1.99 ms, 14 of 5   2.02 ms,
 //                                           8 of 8                 1.94 ms
-// A launch that such groups leave with less than 1.5 tasks per resident warp takes groups of at least 2
+// A launch that such groups leave with less than 1.8 tasks per resident warp takes groups of at least 2
 // strata, and one still below 0.5 single strata; at 16 spp, groups of at least 4 / 2 / 1 strata:
 //   64x48 quads 0.330 / 0.236 / 0.208 ms, box room 0.177 / 0.134 / 0.117  (0.1 / 0.2 / 0.4 tasks a warp)
 //   128x128 quads 0.484 / 0.371, spheres 0.198 / 0.146, mesh 0.585 / 0.486        (0.5 / 1.0)
@@ -337,7 +339,7 @@ RenderGroups render_groups(const RenderDev& R) {
         groups = ((uint64_t)LUM_SMALL_FRAME_TASKS * warps + R.n_tasks - 1) / R.n_tasks;
         const uint64_t n = R.n_tasks;
         uint64_t least = LUM_MIN_GROUP_STRATA;
-        if (2 * n * (n_st / least) < 3 * warps) least = LUM_MIN_GROUP_STRATA / 2;
+        if (5 * n * (n_st / least) < 9 * warps) least = LUM_MIN_GROUP_STRATA / 2;
         if (2 * n * (n_st / least) < warps) least = 1;
         groups = std::min<uint64_t>(groups, std::max<uint64_t>(1, n_st / least));
         const uint64_t wide = n_st / LUM_PREF_GROUP_STRATA;   // groups of the preferred size
@@ -400,11 +402,13 @@ static cudaError_t launch_render_t(const SceneDev& S, const RenderDev& R, float*
     const bool nee = COUNT || S.n_lights > 0;
     const bool sph = !COUNT && !R.ext && S.spheres_basic;
     const int cls = (COUNT || R.ext || sph) ? (int)CLS_ALL : S.cls;
-    const bool many = !COUNT && S.n_prims >= (cls == CLS_MESH ? kManyTriangles : kManyPrims);
+    const bool many = !COUNT && S.n_prims >= many_prims(cls);
     auto kernel = R.ext && S.n_big > 0 ? (nee ? k_render<COUNT, true, true, false, CLS_GROUND>
                                               : k_render<COUNT, true, COUNT, false, CLS_GROUND>)
                 : R.ext ? (nee ? k_render<COUNT, true, true, false> : k_render<COUNT, true, COUNT, false>)
                 : sph   ? (nee ? k_render<COUNT, false, true, !COUNT> : k_render<COUNT, false, COUNT, !COUNT>)
+                : cls == CLS_QUAD && many ? (nee ? k_render<COUNT, false, true, false, CLS_QUAD_MANY>
+                                                 : k_render<COUNT, false, COUNT, false, CLS_QUAD_MANY>)
                 : cls == CLS_QUAD ? (nee ? k_render<COUNT, false, true, false, CLS_QUAD>
                                          : k_render<COUNT, false, COUNT, false, CLS_QUAD>)
                 : cls == CLS_MESH && many ? (nee ? k_render<COUNT, false, true, false, CLS_MESH_MANY>

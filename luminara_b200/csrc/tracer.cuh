@@ -290,17 +290,23 @@ enum : int {
     CLS_QUAD = 1,   // quads (rects, boxes) with rect lights (box room, quad scenes)
     CLS_MESH = 2,   // triangles, disks and media with disk and rect lights (meshes)
     CLS_GROUND = 3, // CLS_ALL, and big spheres apart from the BVH (SceneDev::n_big)
-    CLS_MANY = 4,   // CLS_ALL and CLS_MESH for large scenes (kManyPrims, kManyTriangles): their warps turn to
-    CLS_MESH_MANY = 5   // the leaves once at most two lanes still look for one (walk_warp)
+    CLS_MANY = 4,   // CLS_ALL, CLS_MESH and CLS_QUAD for large scenes (many_prims): their warps turn to the
+    CLS_MESH_MANY = 5,   // leaves once at most two lanes still look for one (walk_warp)
+    CLS_QUAD_MANY = 6
 };
 // From these sizes a walk is long enough that the last lanes' search for a leaf costs the others more
-// than turning to the leaves early does.  No lane against two, 64 spp: mesh of 20k triangles 6.40 /
-// 6.50 ms, 82k 6.94 / 6.95, 328k 7.49 / 7.33, 1.3 M (1080p, 16 spp) 16.7 / 16.1; general scenes of 3k
-// 15.7 / 15.8, 10k 20.6 / 20.5, 30k 24.5 / 23.9; 30 to 300 primitives lose 2-4%.  One lane or three gave
-// less at the large end.
-constexpr int kManyPrims = 16384, kManyTriangles = 65536;
+// than turning to the leaves early does.  No lane against two: mesh of 1.3 M triangles (1080p, 16
+// spp) 16.7 / 15.6 ms, twelve mixed scenes, two above 20k primitives 146.5 / 141.3, 1,004 quads 7.52 / 7.30; below them
+// the box room (18 quads) 1.625 / 1.655, a mesh of 1,280 triangles 5.21 / 5.39, mixed scenes of 30 to
+// 300 primitives 2-4% slower, 20k triangles 1.5%; 3k to 10k mixed primitives and 82k triangles within
+// 1%.  Four lanes gave 2% less on the mesh; ratios of waiting to searching lanes (4, 8, 14) no more.
+__host__ constexpr int many_prims(int cls) {
+    return cls == CLS_MESH ? 65536 : cls == CLS_QUAD ? 512 : 16384;
+}
 template <int CLS>
-__host__ __device__ constexpr int cls_slack() { return CLS == CLS_MANY || CLS == CLS_MESH_MANY ? 2 : 0; }
+__host__ __device__ constexpr bool cls_is_quad() { return CLS == CLS_QUAD || CLS == CLS_QUAD_MANY; }
+template <int CLS>
+__host__ __device__ constexpr int cls_slack() { return CLS == CLS_MANY || CLS == CLS_MESH_MANY || CLS == CLS_QUAD_MANY ? 2 : 0; }
 template <int CLS>
 __host__ __device__ constexpr bool cls_is_mesh() { return CLS == CLS_MESH || CLS == CLS_MESH_MANY; }
 template <int CLS>
@@ -314,15 +320,15 @@ __host__ __device__ constexpr bool cls_is_all() { return CLS == CLS_ALL || CLS =
 // sphere field, bound by issue, runs 4-6% slower that way and keeps them unrolled, as does the
 // quad class (box room 1% slower rolled).
 template <int CLS, bool SPH = false>
-constexpr int philox_unroll() { return CLS == CLS_QUAD || SPH ? 10 : 2; }
+constexpr int philox_unroll() { return CLS == CLS_QUAD || CLS == CLS_QUAD_MANY || SPH ? 10 : 2; }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_prim(int type) {
-    return cls_is_all<CLS>() || (CLS == CLS_QUAD && type == PT_QUAD) ||
+    return cls_is_all<CLS>() || (cls_is_quad<CLS>() && type == PT_QUAD) ||
            (cls_is_mesh<CLS>() && (type == PT_TRIANGLE || type == PT_DISK || type == PT_FOG_SPHERE || type == PT_FOG_BOX));
 }
 template <int CLS>
 __host__ __device__ constexpr bool cls_has_light(int kind) {   // 1 sphere, 2 rect, 3 disk
-    return cls_is_all<CLS>() || (CLS == CLS_QUAD && kind == 2) || (cls_is_mesh<CLS>() && (kind == 2 || kind == 3));
+    return cls_is_all<CLS>() || (cls_is_quad<CLS>() && kind == 2) || (cls_is_mesh<CLS>() && (kind == 2 || kind == 3));
 }
 
 // One primitive test; updates the closest hit when t is within [tmin, hit.t].  The record carries
@@ -346,7 +352,7 @@ __device__ __forceinline__ bool test_prim(const SceneDev& S, int i, const Ray& r
         }
         return false;
     }
-    if constexpr (CLS == CLS_QUAD && !COUNT) {   // every primitive is a quad
+    if constexpr (cls_is_quad<CLS>() && !COUNT) {   // every primitive is a quad
         const float4 b = ldp(S, i, 1), c = ldp(S, i, 2), d = ldp(S, i, 3);
         if (hit_quad(a, b, c, d, ray, tmin, hit.t, t)) { hit.t = t; hit.prim = i; return true; }
         return false;
@@ -382,7 +388,7 @@ __device__ __forceinline__ bool test_prim(const SceneDev& S, int i, const Ray& r
         }
         default: {
             if constexpr (!cls_has_prim<CLS>(PT_FOG_BOX)) return false;
-            const bool fog_hit = CLS != CLS_QUAD ? hit_fog_cold(type, a, b, c, ray, tmin, hit.t, t)
+            const bool fog_hit = !cls_is_quad<CLS>() ? hit_fog_cold(type, a, b, c, ray, tmin, hit.t, t)
                                                  : hit_fog(type, a, b, c, ray, tmin, hit.t, t);
             if (fog_hit) { hit.t = t; hit.prim = i; return true; }
             return false;
@@ -576,11 +582,12 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
                 visit_children(en0, ex0, en1, ex1, link.x, link.y, node, leaf, sp, limit, stride, err);
             }
             // on while some lane that can walk has no leaf yet
-            // (builds for large scenes: while more than kSlack such lanes are left)
+            // (builds for large scenes: while more than kSlack such lanes are left, or none holds a leaf)
             const bool on = (unsigned)node < (unsigned)kSentinel && leaf == 0;
             constexpr int kSlack = cls_slack<CLS>();
             if constexpr (kSlack > 0) {
-                if (__popc(__ballot_sync(full, on)) <= kSlack) break;
+                const unsigned left = __ballot_sync(full, on);
+                if (left == 0 || (__popc(left) <= kSlack && __any_sync(full, leaf < 0))) break;
             } else {
                 if (!__any_sync(full, on)) break;
             }
