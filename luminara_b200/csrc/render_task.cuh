@@ -79,7 +79,7 @@ __device__ __forceinline__ void path_step(const SceneDev& S, const RenderDev& R,
         found = false;
     }
     constexpr unsigned full = 0xffffffffu;
-    const bool done = walk_warp<COUNT, SPH, SUSPEND, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err, act, fresh,
+    const bool done = walk_warp<COUNT, SPH, SPH ? SUSPEND / 2 : SUSPEND, CLS>(S, r, 0.001f, shadow, h, found, tv, stack, err, act, fresh,
                                                              tally);
     walking = act && !done;
     __syncwarp(full);   // the lanes shade together

@@ -636,13 +636,12 @@ __device__ __forceinline__ bool walk_warp(const SceneDev& S, const Ray& ray, flo
     return true;
 }
 
-// LUM_SUSPEND_LANES, the SUSPEND of the persistent kernels' walks: lanes still walking the BVH
-// when at most that many of the warp are left keep their place and let the finished lanes shade
-// and start new rays first (walk_warp); 0 = every walk runs to its end before any lane
-// shades.  Measured on B200 against 0 (kernel time per frame, images
-// identical): 4 / 8 / 16 lanes gave the sphere field 101.7 -> 91.1 / 91.9 / 92.4 ms, the box room
-// 2.57 -> 2.40 / 2.29 / 2.23 ms, the quad scene 13.6 -> 11.5 / 11.4 / 11.8 ms and the dense mesh
-// 238.4 -> 200.6 / 198.3 / 199.7 ms.
+// LUM_SUSPEND_LANES, the SUSPEND of the persistent kernels' walks (half of it in the sphere class):
+// lanes still walking the BVH when at most that many of the warp are left keep their place and let
+// the finished lanes shade and start new rays first (walk_warp); 0 = every walk runs to its end
+// before any lane shades.  Measured on B200 with warp-convergent walks (kernel time per frame,
+// images identical), 4 / 8 / 12 lanes: dense mesh 17.2 / 16.7 / 16.8 ms, quads 7.69 / 7.60 / 7.68, mixed
+// scenes 147.4 / 145.4 / 145.3, sphere field 18.5 / 18.6 / 19.2 (2 lanes 18.5).
 #ifndef LUM_SUSPEND_LANES
 #define LUM_SUSPEND_LANES 8
 #endif
