@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(kSweepThreads, 5) k_sweep(SceneDev S, RenderDe
 
 namespace {
 
-// Vertex staging of one chunk: within what the pool keeps for reuse, with room for the scenes.
+// Vertex staging of one chunk: within what its pool keeps for reuse.
 constexpr size_t kStagingBytes = (size_t)3584 << 20;
 
 lum_status adj_cuda(cudaError_t e, const char* what) {
@@ -879,7 +879,7 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
     if (px == 0 || R.s_end <= R.s_begin || n_mat == 0 || R.max_depth == 0) return LUM_OK;
     // Paths are replayed a chunk of tiles at a time into a staging buffer of vertex records
     // (bounded, at most kStagingBytes or a quarter of free device memory), then swept.  The buffer
-    // comes from the scenes' pool and goes back to it: allocating and freeing 7.2 GB took 5-20 ms per
+    // comes from the staging pool and goes back to it: allocating and freeing 7.2 GB took 5-20 ms per
     // call on B200.
     const uint32_t n_st = R.s_end - R.s_begin;
     const size_t per_tile = (size_t)32 * n_st * (sizeof(adj::PathHead) + (size_t)R.max_depth * sizeof(adj::Vert));

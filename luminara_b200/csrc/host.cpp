@@ -633,31 +633,47 @@ namespace {
 constexpr int kPoolDevices = 64;
 constexpr uint64_t kPoolKeepBytes = 4ull << 30;
 
-lum_status scene_pool(int dev, cudaMemPool_t* out) {
+// The adjoint's staging has a pool of its own: beside the scenes' buffers, whose small blocks split
+// what a call gave back, its few GiB would be allocated again and trimmed again (quads 512x512: 14 or
+// 22 ms per call).  It keeps what one call staged for the next one's, of this scene or another (an
+// optimiser makes a scene per step; allocating 3.5 GB afresh took 22 ms), and gives it back when a
+// scene's allocation finds no memory.
+enum : int { POOL_SCENES = 0, POOL_STAGING = 1 };
+
+lum_status scene_pool(int dev, cudaMemPool_t* out, int which = POOL_SCENES) {
     static std::mutex mu;
-    static cudaMemPool_t pools[kPoolDevices] = {};
+    static cudaMemPool_t pools[2][kPoolDevices] = {};
     if (dev < 0 || dev >= kPoolDevices) return fail(LUM_ERR_TOO_LARGE, "device ordinal above 63");
     std::lock_guard<std::mutex> lk(mu);
-    if (!pools[dev]) {
+    if (!pools[which][dev]) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
-        CU(cudaMemPoolCreate(&pools[dev], &props), "cudaMemPoolCreate");
+        CU(cudaMemPoolCreate(&pools[which][dev], &props), "cudaMemPoolCreate");
         uint64_t keep = kPoolKeepBytes;
-        CU(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+        CU(cudaMemPoolSetAttribute(pools[which][dev], cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
     }
-    *out = pools[dev];
+    *out = pools[which][dev];
     return LUM_OK;
 }
 
 // Pool allocation ordered on the scene's stream; `sync` waits for it, so that the memory can be
 // used from any stream.
-lum_status pool_alloc(lum_scene* s, void** ptr, size_t bytes, bool sync = true) {
+lum_status pool_alloc(lum_scene* s, void** ptr, size_t bytes, bool sync = true, int which = POOL_SCENES) {
     cudaMemPool_t pool = nullptr;
-    lum_status st = scene_pool(s->device, &pool);
+    lum_status st = scene_pool(s->device, &pool, which);
     if (st != LUM_OK) return st;
-    CU(cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream), "cudaMallocFromPoolAsync");
+    cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream);
+    if (e == cudaErrorMemoryAllocation) {   // both pools' idle memory back to the driver, once more
+        cudaGetLastError();
+        for (int p : {POOL_SCENES, POOL_STAGING}) {
+            cudaMemPool_t idle = nullptr;
+            if (scene_pool(s->device, &idle, p) == LUM_OK) cudaMemPoolTrimTo(idle, 0);
+        }
+        e = cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream);
+    }
+    CU(e, "cudaMallocFromPoolAsync");
     if (sync) CU(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
     return LUM_OK;
 }
@@ -1448,7 +1464,9 @@ lum_status prepare_render(lum_scene* s, const lum_render_params* params, SceneDe
     return LUM_OK;
 }
 
-lum_status scratch_alloc(lum_scene* s, void** ptr, size_t bytes) { return pool_alloc(s, ptr, bytes, false); }
+lum_status scratch_alloc(lum_scene* s, void** ptr, size_t bytes) {
+    return pool_alloc(s, ptr, bytes, false, POOL_STAGING);
+}
 
 void scratch_free(lum_scene* s, void* ptr) { cudaFreeAsync(ptr, s->stream); }
 

@@ -772,7 +772,8 @@ struct TableSlot {
     ByteTable T;
 };
 
-static ByteTable byte_table(int kind, double gamma) {
+// build false: only a table that is there already.
+static ByteTable byte_table(int kind, double gamma, bool build = true) {
     static std::mutex mu;
     static std::vector<TableSlot> slots;
     int dev = 0;
@@ -787,6 +788,7 @@ static ByteTable byte_table(int kind, double gamma) {
         ++used;
     }
     TableSlot sl{dev, kind, gb, ByteTable{nullptr, nullptr, 0, 0}};
+    if (!build) return sl.T;
     std::vector<unsigned long long> ent;
     std::vector<uint32_t> ent32;
     void *base = nullptr, *base32 = nullptr;
@@ -832,7 +834,13 @@ cudaError_t launch_tonemap(const float* hdr, uint32_t w, uint32_t h, const lum_t
     }
     const tone::Chain C = tone::make_chain(tm);
     const tone::ByteTable T = C.extra ? tone::ByteTable{nullptr, nullptr, 0, 0} : tone::byte_table(tm.tone_map, tm.gamma);
-    const tone::ByteTable G = C.extra && !tm.dither ? tone::byte_table(tm.tone_map, tm.gamma) : tone::ByteTable{nullptr, nullptr, 0, 0};
+    tone::ByteTable G{nullptr, nullptr, 0, 0};   // of the graded kernel
+    if (C.extra && !tm.dither && vec) {
+        // a table's upload cannot be captured: without one the graded chain takes k_tonemap there
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();
+        G = tone::byte_table(tm.tone_map, tm.gamma, capture == cudaStreamCaptureStatusNone);
+    }
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

@@ -160,3 +160,22 @@ def test_graded_chain_over_ragged_tiles_and_rare_values(chain):
         torch.cuda.synchronize()
         with np.errstate(all="ignore"):
             compare(d_out.cpu().numpy(), OT.tonemap(img, chain))
+
+
+def test_graded_chain_can_be_captured_before_its_table_exists():
+    """The first call of a graded chain inside a stream capture records kernels only (its byte table is
+    not uploaded there), and the replayed graph gives the bytes of a direct call."""
+    import torch
+    img = hdr_image(40, 52, 1)
+    tm = tm_config({"saturation": 1.4, "gamma": 1.9371})                  # a gamma no other test uses
+    d_hdr = torch.from_numpy(img).cuda()
+    a, b = (torch.zeros((40, 52, 4), dtype=torch.uint8, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        L.tonemap_device(d_hdr.data_ptr(), 52, 40, tm, 0, a.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    graph.replay()
+    L.tonemap_device(d_hdr.data_ptr(), 52, 40, tm, 0, b.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    compare(a.cpu().numpy(), b.cpu().numpy())
+    compare(b.cpu().numpy(), OT.tonemap(img, {"saturation": 1.4, "gamma": 1.9371}))
