@@ -459,8 +459,8 @@ lum_status lum_forward(lum_scene* scene, const lum_render_params* params, float*
  * the expected image; visibility changes are not differentiated.  max_depth <= 16.  Pixels
  * whose dL/d(image) is zero are not replayed.  The call stages one chunk of replayed paths at
  * a time in device memory (at most 3.5 GiB or a quarter of the free memory, 48 + 64 * max_depth
- * bytes per path), from a second pool that keeps up to 4 GiB for the next call and gives it
- * back when a scene's allocation finds no memory. */
+ * bytes per path).  The largest such buffer (up to 4 GiB per device) is kept for the next call
+ * and given back when an allocation of this library finds no memory. */
 lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const float* dL_dimage,
                         const int32_t* light_material, float* d_albedo, float* d_roughness, float* d_emission,
                         lum_stats* stats);

@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(kSweepThreads, 5) k_sweep(SceneDev S, RenderDe
 
 namespace {
 
-// Vertex staging of one chunk: within what its pool keeps for reuse.
+// Vertex staging of one chunk: within what scratch_free keeps for reuse.
 constexpr size_t kStagingBytes = (size_t)3584 << 20;
 
 lum_status adj_cuda(cudaError_t e, const char* what) {
@@ -879,7 +879,7 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
     if (px == 0 || R.s_end <= R.s_begin || n_mat == 0 || R.max_depth == 0) return LUM_OK;
     // Paths are replayed a chunk of tiles at a time into a staging buffer of vertex records
     // (bounded, at most kStagingBytes or a quarter of free device memory), then swept.  The buffer
-    // comes from the staging pool and goes back to it: allocating and freeing 7.2 GB took 5-20 ms per
+    // is kept for the next call: allocating and freeing 7.2 GB took 5-20 ms per
     // call on B200.
     const uint32_t n_st = R.s_end - R.s_begin;
     const size_t per_tile = (size_t)32 * n_st * (sizeof(adj::PathHead) + (size_t)R.max_depth * sizeof(adj::Vert));
@@ -897,7 +897,8 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
                  o_heads = o_wc + al(sizeof(WorkCounters)), o_verts = o_heads + al(bytes_heads),
                  total = o_verts + al(bytes_verts);
     char* buf = nullptr;
-    if ((st = scratch_alloc(scene, (void**)&buf, total)) != LUM_OK) return st;
+    size_t buf_bytes = total;
+    if ((st = scratch_alloc(scene, (void**)&buf, &buf_bytes)) != LUM_OK) return st;
     cudaError_t e = cudaSuccess;
     float* d_img = (float*)buf;
     float* d_g = (float*)(buf + o_g);
@@ -981,7 +982,7 @@ lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const
     if (ok) cudaEventElapsedTime(&ms, ev0, ev1);
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
-    scratch_free(scene, buf);
+    scratch_free(scene, buf, buf_bytes);
     if (!ok) return adj_cuda(e, "lum_backward");
     std::memcpy(d_albedo, hg.data(), sizeof(float) * 3 * n_mat);
     std::memcpy(d_roughness, hg.data() + 3 * n_mat, sizeof(float) * n_mat);

@@ -633,44 +633,61 @@ namespace {
 constexpr int kPoolDevices = 64;
 constexpr uint64_t kPoolKeepBytes = 4ull << 30;
 
-// The adjoint's staging has a pool of its own: beside the scenes' buffers, whose small blocks split
-// what a call gave back, its few GiB would be allocated again and trimmed again (quads 512x512: 14 or
-// 22 ms per call).  It keeps what one call staged for the next one's, of this scene or another (an
-// optimiser makes a scene per step; allocating 3.5 GB afresh took 22 ms), and gives it back when a
-// scene's allocation finds no memory.
-enum : int { POOL_SCENES = 0, POOL_STAGING = 1 };
-
-lum_status scene_pool(int dev, cudaMemPool_t* out, int which = POOL_SCENES) {
+lum_status scene_pool(int dev, cudaMemPool_t* out) {
     static std::mutex mu;
-    static cudaMemPool_t pools[2][kPoolDevices] = {};
+    static cudaMemPool_t pools[kPoolDevices] = {};
     if (dev < 0 || dev >= kPoolDevices) return fail(LUM_ERR_TOO_LARGE, "device ordinal above 63");
     std::lock_guard<std::mutex> lk(mu);
-    if (!pools[which][dev]) {
+    if (!pools[dev]) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
-        CU(cudaMemPoolCreate(&pools[which][dev], &props), "cudaMemPoolCreate");
+        CU(cudaMemPoolCreate(&pools[dev], &props), "cudaMemPoolCreate");
         uint64_t keep = kPoolKeepBytes;
-        CU(cudaMemPoolSetAttribute(pools[which][dev], cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+        CU(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
     }
-    *out = pools[which][dev];
+    *out = pools[dev];
     return LUM_OK;
+}
+
+// The adjoint's staging buffer that no call uses, one per device and at most kPoolKeepBytes: the
+// next call, of this scene or another (an optimiser makes a scene per step), takes it.  In a
+// stream-ordered pool a few GiB were in some processes allocated and trimmed again by every call
+// (quads 512x512: 13 or 25 ms per call, in the scenes' pool 14 or 22).
+struct IdleBuffer {
+    std::mutex mu;
+    void* ptr = nullptr;
+    size_t bytes = 0;
+};
+
+IdleBuffer* idle_buffer(int dev) {
+    static IdleBuffer idle[kPoolDevices];
+    return dev >= 0 && dev < kPoolDevices ? &idle[dev] : nullptr;
+}
+
+// What is kept for reuse goes back to the driver.
+void give_back_idle(int dev) {
+    cudaMemPool_t pool = nullptr;
+    if (scene_pool(dev, &pool) == LUM_OK) cudaMemPoolTrimTo(pool, 0);
+    if (IdleBuffer* idle = idle_buffer(dev)) {
+        std::lock_guard<std::mutex> lk(idle->mu);
+        if (idle->ptr) cudaFree(idle->ptr);
+        idle->ptr = nullptr;
+        idle->bytes = 0;
+    }
 }
 
 // Pool allocation ordered on the scene's stream; `sync` waits for it, so that the memory can be
 // used from any stream.
-lum_status pool_alloc(lum_scene* s, void** ptr, size_t bytes, bool sync = true, int which = POOL_SCENES) {
+lum_status pool_alloc(lum_scene* s, void** ptr, size_t bytes, bool sync = true) {
     cudaMemPool_t pool = nullptr;
-    lum_status st = scene_pool(s->device, &pool, which);
+    lum_status st = scene_pool(s->device, &pool);
     if (st != LUM_OK) return st;
     cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream);
-    if (e == cudaErrorMemoryAllocation) {   // both pools' idle memory back to the driver, once more
+    if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        for (int p : {POOL_SCENES, POOL_STAGING}) {
-            cudaMemPool_t idle = nullptr;
-            if (scene_pool(s->device, &idle, p) == LUM_OK) cudaMemPoolTrimTo(idle, 0);
-        }
+        give_back_idle(s->device);
         e = cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream);
     }
     CU(e, "cudaMallocFromPoolAsync");
@@ -1464,11 +1481,39 @@ lum_status prepare_render(lum_scene* s, const lum_render_params* params, SceneDe
     return LUM_OK;
 }
 
-lum_status scratch_alloc(lum_scene* s, void** ptr, size_t bytes) {
-    return pool_alloc(s, ptr, bytes, false, POOL_STAGING);
+lum_status scratch_alloc(lum_scene* s, void** ptr, size_t* bytes) {
+    if (IdleBuffer* idle = idle_buffer(s->device)) {
+        std::lock_guard<std::mutex> lk(idle->mu);
+        if (idle->ptr && idle->bytes >= *bytes) {
+            *ptr = idle->ptr;
+            *bytes = idle->bytes;
+            idle->ptr = nullptr;
+            idle->bytes = 0;
+            return LUM_OK;
+        }
+    }
+    cudaError_t e = cudaMalloc(ptr, *bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        give_back_idle(s->device);
+        e = cudaMalloc(ptr, *bytes);
+    }
+    CU(e, "cudaMalloc");
+    return LUM_OK;
 }
 
-void scratch_free(lum_scene* s, void* ptr) { cudaFreeAsync(ptr, s->stream); }
+void scratch_free(lum_scene* s, void* ptr, size_t bytes) {
+    cudaStreamSynchronize(s->stream);   // a call that failed may have work in flight
+    IdleBuffer* idle = idle_buffer(s->device);
+    if (idle && bytes <= kPoolKeepBytes) {
+        std::lock_guard<std::mutex> lk(idle->mu);
+        if (bytes > idle->bytes) {
+            std::swap(ptr, idle->ptr);
+            idle->bytes = bytes;
+        }
+    }
+    if (ptr) cudaFree(ptr);
+}
 
 int scene_max_material_kind(const lum_scene* s) { return s ? s->max_mat_kind : 0; }
 

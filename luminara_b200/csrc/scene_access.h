@@ -23,11 +23,11 @@ lum_status prepare_render(lum_scene* s, const lum_render_params* params, SceneDe
 lum_status scene_view(lum_scene* s, const lum_render_params* params, SceneDev& dev, RenderDev& R, int& device);
 // Largest LUM_MAT_* kind among the scene's materials (0 when it has none).
 int scene_max_material_kind(const lum_scene* s);
-// Device memory of one call from the staging pool, ordered on the scene's stream; freed memory stays
-// in the pool (up to its bound) for the next call, and goes back to the driver when a scene's
-// allocation finds no memory.
-lum_status scratch_alloc(lum_scene* s, void** ptr, size_t bytes);
-void scratch_free(lum_scene* s, void* ptr);
+// Device memory of one call, at least `*bytes` (set to its size).  scratch_free waits for the scene's
+// stream; the largest freed buffer (up to 4 GiB) is kept per device for the next call, and goes back
+// to the driver when an allocation finds no memory.
+lum_status scratch_alloc(lum_scene* s, void** ptr, size_t* bytes);
+void scratch_free(lum_scene* s, void* ptr, size_t bytes);
 // The mutex that serialises calls on one scene handle (held by every entry point that reads
 // the scene's device buffers).
 std::mutex& scene_mutex(lum_scene* s);
