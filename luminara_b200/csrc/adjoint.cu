@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "pool_index.h"
 #include "scene_access.h"
 #include "tracer.cuh"
 
@@ -623,8 +624,8 @@ __global__ void __launch_bounds__(128, LUM_ADJ_MIN_BLOCKS) k_replay(SceneDev S, 
             for (uint32_t s2 = s_lo; s2 < s_hi; ++s2) heads[slot_base + lane + (size_t)(s2 - R.s_begin) * 32].K = -1;
         const unsigned with = __ballot_sync(kFullMask, replay);
         const uint32_t n_px = __popc(with), n_items = n_px * (s_hi - s_lo);
-        // idx / n_px by a high multiply (idx * n_px < 2^32); 0: one pixel
-        const uint32_t magic = n_px > 1 ? 0xFFFFFFFFu / n_px + 1u : 0u;
+        // at most 32 pixels of kReplayStrata strata: the high multiply serves them all; 0: one pixel
+        const uint32_t magic = pool_magic(n_px, n_items);
         if (replay) s_slot[wid][__popc(with & ((1u << lane) - 1u))] = lane;
         if (lane == 0) s_next[wid] = 0u;
         __syncwarp(kFullMask);

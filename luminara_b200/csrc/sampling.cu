@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "pool_index.h"
 #include "render_task.cuh"
 #include "tracer.cuh"
 
@@ -50,8 +51,10 @@ __device__ __forceinline__ V clamp_sample(V L) {
 // centre sample (n_st = 1, stratum 0).  With acc, each finished path adds its clamped,
 // filter-weighted value to acc[tile pixel] in fixed point (tile_task's sums; the call zeroes
 // acc); without, its clamped sample goes to smp[stratum - st_lo][tile pixel].  One copy of
-// the traversal and shading code serves every kind of tile.
-template <bool EXT, bool NEE, bool SPH, int CLS>
+// the traversal and shading code serves every kind of tile.  SMALL: the pool holds at most a round's
+// kRoundStrata strata of 32 slots, which the high multiply always serves (a time-limited tile's pool
+// holds all its strata, millions of them at the largest sample counts).
+template <bool SMALL, bool EXT, bool NEE, bool SPH, int CLS>
 __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& R, uint32_t x0, uint32_t y0, uint32_t tw,
                             const uint32_t* slot_px, uint32_t n_slots, uint32_t st_lo, uint32_t n_st, bool centre,
                             unsigned long long (*acc)[4], float (*smp)[32][3], uint32_t* next, V* exit_stash,
@@ -61,8 +64,7 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
     if (lane == 0) *next = 0u;
     __syncwarp(kAll);
     const uint32_t n_items = n_slots * n_st;
-    // idx / n_slots by a high multiply (exact for idx * n_slots < 2^32); 0: one slot
-    const uint32_t magic = n_slots > 1 ? 0xFFFFFFFFu / n_slots + 1u : 0u;
+    const uint32_t magic = pool_magic(n_slots, SMALL ? 0 : (uint64_t)n_slots * n_st);
     int state = ST_IDLE;
     uint32_t px = 0, k = 0, pixel = 0;
     Path P;
@@ -74,7 +76,8 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
         if (state == ST_IDLE) {
             const uint32_t idx = atomicAdd(next, 1u);
             if (idx < n_items) {
-                k = magic ? __umulhi(idx, magic) : idx;
+                if constexpr (SMALL) k = magic ? __umulhi(idx, magic) : idx;
+                else k = pool_stratum(idx, n_slots, magic);
                 px = slot_px[idx - k * n_slots];
                 const uint32_t row = tw == 8u ? px >> 3 : px / tw;
                 const uint32_t gi = x0 + px - row * tw + R.crop_x, gj = y0 + row + R.crop_y;
@@ -165,7 +168,7 @@ __global__ void __launch_bounds__(kSampThreads, ADAPTIVE ? 5 : 7) k_render_sampl
             if (active) s_slot[wid][__popc(act & ((1u << lane) - 1u))] = lane;
             const uint32_t st_lo = expired ? 0u : ADAPTIVE ? lo : R.s_begin;
             const uint32_t n_st = expired ? 1u : ADAPTIVE ? min(kRoundStrata, total - lo) : R.s_end - R.s_begin;
-            sample_pool<EXT, NEE, SPH, CLS>(S, R, x0, y0, tw, s_slot[wid], __popc(act), st_lo, n_st, expired != 0,
+            sample_pool<ADAPTIVE, EXT, NEE, SPH, CLS>(S, R, x0, y0, tw, s_slot[wid], __popc(act), st_lo, n_st, expired != 0,
                                             fixed_sums ? s_acc[ADAPTIVE ? 0 : wid] : nullptr, s_smp[wid], &s_next[wid],
                                             s_exit[EXT ? wid : 0], stack, err, nseg, nsh);
             if (active) {
