@@ -35,6 +35,7 @@
 #include "../../include/luminara_gpu.h"
 #include "kernels.h"
 #include "scene_access.h"
+#include "table_cache.h"
 
 namespace lum {
 namespace tone {
@@ -307,7 +308,6 @@ __device__ __forceinline__ uint32_t tone_gamma_fast(float v, float exposure32, d
 constexpr int kTabShift = 45;                                  // 52 - 7 mantissa bits
 constexpr unsigned long long kTabLowMask = (1ull << kTabShift) - 1ull;
 constexpr int kTabMaxEntries = 4096;                           // nb + 2 per table
-constexpr int kTabSlots = 16;                                  // (tone curve, gamma) pairs per device
 
 struct ByteTable {
     const unsigned long long* tab;   // device address of the slot, or null: no table
@@ -315,6 +315,7 @@ struct ByteTable {
     long long k0;                    // bucket key of entry 1
     int nb;                          // buckets with an entry of their own
 };
+constexpr int kTabSlots = TableCache<ByteTable>::kSlots;       // (tone curve, gamma) pairs per device
 
 static __device__ __align__(256) unsigned long long g_byte_tables[kTabSlots][kTabMaxEntries];
 // 32-bit entries for a power-of-two exposure, where x's bits below the bucket are the low 16 bits m
@@ -765,53 +766,47 @@ static bool build_byte_table(int kind, double gamma, std::vector<unsigned long l
     return true;
 }
 
-// One table per (device, tone curve, gamma), uploaded once into a slot of g_byte_tables.
-struct TableSlot {
-    int device, kind;
-    long long gamma_bits;
-    ByteTable T;
-};
-
-// build false: only a table that is there already.
-static ByteTable byte_table(int kind, double gamma, bool build = true) {
+// One table per (device, tone curve, gamma), uploaded once into a slot of g_byte_tables.  graded: for a
+// chain with optional steps.  build false: only a table that is there already.
+static ByteTable byte_table(int kind, double gamma, bool graded, bool build = true) {
     static std::mutex mu;
-    static std::vector<TableSlot> slots;
+    static TableCache<ByteTable> cache;
+    const ByteTable none{nullptr, nullptr, 0, 0};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return ByteTable{nullptr, nullptr, 0, 0};
+    if (cudaGetDevice(&dev) != cudaSuccess) return none;
     if (!(gamma > 0.0)) gamma = 0.0;
     const long long gb = dbits(gamma);
     std::lock_guard<std::mutex> lk(mu);
-    int used = 0;
-    for (const TableSlot& sl : slots) {
-        if (sl.device != dev) continue;
-        if (sl.kind == kind && sl.gamma_bits == gb) return sl.T;
-        ++used;
-    }
-    TableSlot sl{dev, kind, gb, ByteTable{nullptr, nullptr, 0, 0}};
-    if (!build) return sl.T;
+    bool known = false;
+    if (const ByteTable* t = cache.find(dev, kind, gb, &known)) return *t;
+    const int slot = cache.free_slot(dev, graded);
+    if (known || !build || slot < 0) return none;
+    ByteTable T = none;
     std::vector<unsigned long long> ent;
     std::vector<uint32_t> ent32;
-    void *base = nullptr, *base32 = nullptr;
-    if (used < kTabSlots && build_byte_table(kind, gamma, ent, sl.T.k0, sl.T.nb)) {
-        for (const unsigned long long e : ent) {
-            const unsigned long long thr = e & (2ull * kTabLowMask + 1ull);
-            const uint32_t t16 = thr > kTabLowMask ? 65536u : (uint32_t)((thr + (1ull << 29) - 1) >> 29);
-            ent32.push_back(((uint32_t)(e >> 56) << 16) + 65536u - t16);
-        }
-        if (cudaGetSymbolAddress(&base, g_byte_tables) == cudaSuccess &&
-            cudaGetSymbolAddress(&base32, g_byte_tables32) == cudaSuccess &&
-            cudaMemcpyToSymbol(g_byte_tables, ent.data(), ent.size() * sizeof(unsigned long long),
-                               (size_t)used * kTabMaxEntries * sizeof(unsigned long long)) == cudaSuccess &&
-            cudaMemcpyToSymbol(g_byte_tables32, ent32.data(), ent32.size() * sizeof(uint32_t),
-                               (size_t)used * kTabMaxEntries * sizeof(uint32_t)) == cudaSuccess) {
-            sl.T.tab = static_cast<const unsigned long long*>(base) + (size_t)used * kTabMaxEntries;
-            sl.T.tab32 = static_cast<const uint32_t*>(base32) + (size_t)used * kTabMaxEntries;
-        }
+    if (!build_byte_table(kind, gamma, ent, T.k0, T.nb)) {
+        cache.add_failed(dev, kind, gb);
+        return none;
     }
-    cudaGetLastError();
-    if (!sl.T.tab) sl.kind = -1 - kind;                         // remembered as "no table"
-    slots.push_back(sl);
-    return sl.T;
+    for (const unsigned long long e : ent) {
+        const unsigned long long thr = e & (2ull * kTabLowMask + 1ull);
+        const uint32_t t16 = thr > kTabLowMask ? 65536u : (uint32_t)((thr + (1ull << 29) - 1) >> 29);
+        ent32.push_back(((uint32_t)(e >> 56) << 16) + 65536u - t16);
+    }
+    void *base = nullptr, *base32 = nullptr;
+    if (cudaGetSymbolAddress(&base, g_byte_tables) != cudaSuccess ||
+        cudaGetSymbolAddress(&base32, g_byte_tables32) != cudaSuccess ||
+        cudaMemcpyToSymbol(g_byte_tables, ent.data(), ent.size() * sizeof(unsigned long long),
+                           (size_t)slot * kTabMaxEntries * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMemcpyToSymbol(g_byte_tables32, ent32.data(), ent32.size() * sizeof(uint32_t),
+                           (size_t)slot * kTabMaxEntries * sizeof(uint32_t)) != cudaSuccess) {
+        cudaGetLastError();                                     // the next call tries again
+        return none;
+    }
+    T.tab = static_cast<const unsigned long long*>(base) + (size_t)slot * kTabMaxEntries;
+    T.tab32 = static_cast<const uint32_t*>(base32) + (size_t)slot * kTabMaxEntries;
+    cache.add(dev, kind, gb, slot, T);
+    return T;
 }
 
 }  // namespace tone
@@ -833,13 +828,13 @@ cudaError_t launch_tonemap(const float* hdr, uint32_t w, uint32_t h, const lum_t
         partials = scratch;
     }
     const tone::Chain C = tone::make_chain(tm);
-    const tone::ByteTable T = C.extra ? tone::ByteTable{nullptr, nullptr, 0, 0} : tone::byte_table(tm.tone_map, tm.gamma);
+    const tone::ByteTable T = C.extra ? tone::ByteTable{nullptr, nullptr, 0, 0} : tone::byte_table(tm.tone_map, tm.gamma, false);
     tone::ByteTable G{nullptr, nullptr, 0, 0};   // of the graded kernel
     if (C.extra && !tm.dither && vec) {
         // a table's upload cannot be captured: without one the graded chain takes k_tonemap there
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();
-        G = tone::byte_table(tm.tone_map, tm.gamma, capture == cudaStreamCaptureStatusNone);
+        G = tone::byte_table(tm.tone_map, tm.gamma, true, capture == cudaStreamCaptureStatusNone);
     }
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);

@@ -179,3 +179,16 @@ def test_graded_chain_can_be_captured_before_its_table_exists():
     torch.cuda.synchronize()
     compare(a.cpu().numpy(), b.cpu().numpy())
     compare(b.cpu().numpy(), OT.tonemap(img, {"saturation": 1.4, "gamma": 1.9371}))
+
+
+@pytest.mark.parametrize("steps", [{}, {"saturation": 1.2}])
+def test_gammas_without_a_table_and_new_pairs_after_them(steps):
+    """A gamma whose curve fits no byte table (ACES at 4) over many calls, then pairs of their own: the chain's
+    bytes from whichever kernel takes them (which pairs get tables is checked in test_table_cache)."""
+    import torch
+    img = hdr_image(16, 32, 3)
+    d_hdr, d_out = torch.from_numpy(img).cuda(), torch.zeros((16, 32, 4), dtype=torch.uint8, device="cuda")
+    for chain in [{**steps, "gamma": g} for g in [4.0] * 40 + [1.2345, 2.2, 4.0, 1.5]]:
+        L.tonemap_device(d_hdr.data_ptr(), 32, 16, tm_config(chain), 0, d_out.data_ptr())
+        torch.cuda.synchronize()
+        compare(d_out.cpu().numpy(), OT.tonemap(img, chain))
