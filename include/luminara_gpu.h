@@ -578,9 +578,12 @@ void lum_tonemap_default(lum_tonemap_params* out);
  * auto_exposure (may be NULL otherwise; 8-byte aligned).  d_hdr_rgb must be 4-byte aligned,
  * d_rgba may have any alignment (16-byte aligned buffers take the vectorised path).
  * Allocates nothing; does not synchronise, except that the first call on a device for a given
- * (tone_map, gamma) pair without optional steps computes that chain's byte-threshold table on
- * the host (a few milliseconds) and copies it synchronously into a fixed device table (16
- * pairs per device); make that first call outside stream capture. */
+ * (tone_map, gamma) pair -- without optional steps, or with optional steps but no dither on
+ * 16-byte aligned buffers -- computes that chain's byte-threshold table on the host (a few
+ * milliseconds), copies it into a fixed device table on a stream of its own and waits for that
+ * copy.  It may be made while this or another stream is being captured.  A device holds tables
+ * of 16 pairs, and of 8 more first met with optional steps; other pairs, and pairs whose curve
+ * fits no table, take a slower kernel with the same bytes. */
 lum_status lum_tonemap_device(const float* d_hdr_rgb, uint32_t width, uint32_t height,
                               const lum_tonemap_params* tm, void* d_scratch, uint8_t* d_rgba,
                               void* stream);

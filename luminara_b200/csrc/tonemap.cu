@@ -766,9 +766,28 @@ static bool build_byte_table(int kind, double gamma, std::vector<unsigned long l
     return true;
 }
 
+// Copies a table into its slot, on a stream of its own and with this thread's capture mode relaxed: a copy
+// on the default stream would break a stream capture of this thread or, in the global mode, of any.
+template <class T>
+static bool upload_table(T (&symbol)[kTabSlots][kTabMaxEntries], const std::vector<T>& ent, int slot, void** base) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
+    cudaStream_t stream = nullptr;
+    bool ok = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess;
+    if (ok) {
+        ok = cudaGetSymbolAddress(base, symbol) == cudaSuccess &&
+             cudaMemcpyAsync(static_cast<T*>(*base) + (size_t)slot * kTabMaxEntries, ent.data(), ent.size() * sizeof(T),
+                             cudaMemcpyHostToDevice, stream) == cudaSuccess;
+        ok = cudaStreamSynchronize(stream) == cudaSuccess && ok;
+        cudaStreamDestroy(stream);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return ok;
+}
+
 // One table per (device, tone curve, gamma), uploaded once into a slot of g_byte_tables.  graded: for a
-// chain with optional steps.  build false: only a table that is there already.
-static ByteTable byte_table(int kind, double gamma, bool graded, bool build = true) {
+// chain with optional steps.
+static ByteTable byte_table(int kind, double gamma, bool graded) {
     static std::mutex mu;
     static TableCache<ByteTable> cache;
     const ByteTable none{nullptr, nullptr, 0, 0};
@@ -780,7 +799,7 @@ static ByteTable byte_table(int kind, double gamma, bool graded, bool build = tr
     bool known = false;
     if (const ByteTable* t = cache.find(dev, kind, gb, &known)) return *t;
     const int slot = cache.free_slot(dev, graded);
-    if (known || !build || slot < 0) return none;
+    if (known || slot < 0) return none;
     ByteTable T = none;
     std::vector<unsigned long long> ent;
     std::vector<uint32_t> ent32;
@@ -794,12 +813,7 @@ static ByteTable byte_table(int kind, double gamma, bool graded, bool build = tr
         ent32.push_back(((uint32_t)(e >> 56) << 16) + 65536u - t16);
     }
     void *base = nullptr, *base32 = nullptr;
-    if (cudaGetSymbolAddress(&base, g_byte_tables) != cudaSuccess ||
-        cudaGetSymbolAddress(&base32, g_byte_tables32) != cudaSuccess ||
-        cudaMemcpyToSymbol(g_byte_tables, ent.data(), ent.size() * sizeof(unsigned long long),
-                           (size_t)slot * kTabMaxEntries * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemcpyToSymbol(g_byte_tables32, ent32.data(), ent32.size() * sizeof(uint32_t),
-                           (size_t)slot * kTabMaxEntries * sizeof(uint32_t)) != cudaSuccess) {
+    if (!upload_table(g_byte_tables, ent, slot, &base) || !upload_table(g_byte_tables32, ent32, slot, &base32)) {
         cudaGetLastError();                                     // the next call tries again
         return none;
     }
@@ -830,12 +844,7 @@ cudaError_t launch_tonemap(const float* hdr, uint32_t w, uint32_t h, const lum_t
     const tone::Chain C = tone::make_chain(tm);
     const tone::ByteTable T = C.extra ? tone::ByteTable{nullptr, nullptr, 0, 0} : tone::byte_table(tm.tone_map, tm.gamma, false);
     tone::ByteTable G{nullptr, nullptr, 0, 0};   // of the graded kernel
-    if (C.extra && !tm.dither && vec) {
-        // a table's upload cannot be captured: without one the graded chain takes k_tonemap there
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();
-        G = tone::byte_table(tm.tone_map, tm.gamma, true, capture == cudaStreamCaptureStatusNone);
-    }
+    if (C.extra && !tm.dither && vec) G = tone::byte_table(tm.tone_map, tm.gamma, true);
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

@@ -192,3 +192,36 @@ def test_gammas_without_a_table_and_new_pairs_after_them(steps):
         L.tonemap_device(d_hdr.data_ptr(), 32, 16, tm_config(chain), 0, d_out.data_ptr())
         torch.cuda.synchronize()
         compare(d_out.cpu().numpy(), OT.tonemap(img, chain))
+
+
+@pytest.mark.parametrize("steps", [{}, {"saturation": 1.2}])
+@pytest.mark.parametrize("mode", ["global", "thread_local"])
+@pytest.mark.parametrize("blocking", [False, True])
+@pytest.mark.parametrize("own", [False, True])
+def test_first_call_of_a_pair_leaves_stream_captures_whole(steps, mode, blocking, own):
+    """The first call of a (curve, gamma) pair uploads its table.  Made while a stream (one that waits for
+    the default stream, or not) is being captured, it neither breaks the capture nor is broken by it: on a
+    stream beside the captured one it runs at once, on the captured stream it becomes part of the graph."""
+    import ctypes
+
+    import torch
+    chain = {**steps, "gamma": 1.61 + 0.01 * len(steps) + 0.1 * own + (0.2 if mode == "global" else 0.0) + 0.4 * blocking}
+    img = hdr_image(24, 36, 2)
+    d_hdr = torch.from_numpy(img).cuda()
+    out, x = torch.zeros((24, 36, 4), dtype=torch.uint8, device="cuda"), torch.zeros(8, device="cuda")
+    beside = torch.cuda.Stream()
+    captured = None
+    if blocking:
+        handle = ctypes.c_void_p()
+        assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle))) == 0
+        captured = torch.cuda.ExternalStream(handle.value)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=captured, capture_error_mode=mode):
+        x.add_(1.0)
+        stream = torch.cuda.current_stream() if own else beside
+        L.tonemap_device(d_hdr.data_ptr(), 36, 24, tm_config(chain), 0, out.data_ptr(), stream.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (x == 1.0).all()
+    compare(out.cpu().numpy(), OT.tonemap(img, chain))
