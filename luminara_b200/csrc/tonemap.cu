@@ -610,7 +610,8 @@ __global__ void __launch_bounds__(kGradedThreads, kGradedBlocks)
                      const double* __restrict__ partials, uint8_t* __restrict__ rgba, const ByteTable T) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ uint8_t s_before[256], s_after[3][256];
-    __shared__ float s_px[kGradedThreads / 32][96];
+    __shared__ float4 s_px[kGradedThreads / 32][24];   // written so, read as 96 floats
+    static_assert(alignof(decltype(s_px)) == 16, "the stores are 16 bytes wide");
     auto* tab = reinterpret_cast<unsigned long long*>(s_raw);
     const int top = T.nb + 1;
     for (int i = threadIdx.x; i <= top; i += kGradedThreads) tab[i] = __ldg(T.tab + i);
@@ -631,7 +632,7 @@ __global__ void __launch_bounds__(kGradedThreads, kGradedBlocks)
         return (uint32_t)(e >> 56) + (((unsigned long long)b & kTabLowMask) >= (e & (2ull * kTabLowMask + 1ull)) ? 1u : 0u);
     };
     const int lane = threadIdx.x & 31;
-    float* px = s_px[threadIdx.x >> 5];
+    const float* px = reinterpret_cast<const float*>(s_px[threadIdx.x >> 5]);
     const double dw = (double)w, dh = (double)h, rw = 1.0 / dw, rh = 1.0 / dh;
     const uint32_t tiles = (n + 31) / 32, step = gridDim.x * (kGradedThreads / 32), lim = 3 * (n / 4);
     const float4* in = reinterpret_cast<const float4*>(hdr);
@@ -650,7 +651,7 @@ __global__ void __launch_bounds__(kGradedThreads, kGradedBlocks)
     uint32_t t = blockIdx.x * (kGradedThreads / 32) + (threadIdx.x >> 5);
     float4 f = fetch(t);
     for (; t < tiles; t += step) {
-        if (lane < 24) reinterpret_cast<float4*>(px)[lane] = f;
+        if (lane < 24) s_px[threadIdx.x >> 5][lane] = f;
         if (t < tiles - min(tiles, step)) f = fetch(t + step);
         __syncwarp();
         const double r = px[3 * lane], g = px[3 * lane + 1], b = px[3 * lane + 2];
