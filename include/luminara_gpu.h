@@ -335,7 +335,8 @@ lum_status lum_scene_create(const lum_scene_desc* desc, lum_scene** out_scene);
 
 /* Frees the scene's device buffers (back to the device's pool) and stream.  Synchronises the
  * device first, as cudaFree would, so work that other streams still run on the scene
- * finishes before its memory is reused. */
+ * finishes before its memory is reused.  The device's last scene also gives lum_backward's idle
+ * staging buffer back to the driver. */
 lum_status lum_scene_destroy(lum_scene* scene);
 
 /* Number of expanded primitives and BVH nodes (diagnostics). */
@@ -459,8 +460,9 @@ lum_status lum_forward(lum_scene* scene, const lum_render_params* params, float*
  * the expected image; visibility changes are not differentiated.  max_depth <= 16.  Pixels
  * whose dL/d(image) is zero are not replayed.  The call stages one chunk of replayed paths at
  * a time in device memory (at most 3.5 GiB or a quarter of the free memory, 48 + 64 * max_depth
- * bytes per path).  The largest such buffer (up to 4 GiB per device) is kept for the next call
- * and given back when an allocation of this library finds no memory. */
+ * bytes per path).  The largest such buffer (up to 4 GiB per device) is kept for the next call.
+ * It is given back when an allocation of this library finds no memory, and with the last scene
+ * destroyed on the device. */
 lum_status lum_backward(lum_scene* scene, const lum_render_params* params, const float* dL_dimage,
                         const int32_t* light_material, float* d_albedo, float* d_roughness, float* d_emission,
                         lum_stats* stats);

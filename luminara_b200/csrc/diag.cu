@@ -70,8 +70,8 @@ extern "C" lum_status lum_diag_l1_throughput(int32_t pattern, double* gbs) {
     char msg[256];
     const uint32_t iters = 8192;
     float best = 1e30f;
-    if ((e = cudaMalloc(&tab, kTableVec * sizeof(float4))) != cudaSuccess ||
-        (e = cudaMalloc(&out, (size_t)grid * kProbeThreads * sizeof(float))) != cudaSuccess ||
+    if ((e = lum::device_malloc(dev, (void**)&tab, kTableVec * sizeof(float4))) != cudaSuccess ||
+        (e = lum::device_malloc(dev, (void**)&out, (size_t)grid * kProbeThreads * sizeof(float))) != cudaSuccess ||
         (e = cudaMemset(tab, 0, kTableVec * sizeof(float4))) != cudaSuccess ||
         (e = cudaEventCreate(&e0)) != cudaSuccess || (e = cudaEventCreate(&e1)) != cudaSuccess)
         goto done;

@@ -24,6 +24,7 @@
 #include "../../include/luminara_gpu.h"
 #include "bvh_build.h"
 #include "device_scene.h"
+#include "idle_buffer.h"
 #include "kernels.h"
 #include "scene_access.h"
 
@@ -620,6 +621,7 @@ struct lum_scene {
     lum::SceneDev dev{};
     uint32_t n_prims = 0, n_nodes = 0, n_lights = 0, bvh_depth = 0;
     int max_mat_kind = 0;
+    lum::IdleBuffer* idle = nullptr;   // of the device: kept while the device has scenes
     std::mutex mu;
 };
 
@@ -655,27 +657,20 @@ lum_status scene_pool(int dev, cudaMemPool_t* out) {
 // next call, of this scene or another (an optimiser makes a scene per step), takes it.  In a
 // stream-ordered pool a few GiB were in some processes allocated and trimmed again by every call
 // (quads 512x512: 13 or 25 ms per call, in the scenes' pool 14 or 22).
-struct IdleBuffer {
-    std::mutex mu;
-    void* ptr = nullptr;
-    size_t bytes = 0;
-};
-
-IdleBuffer* idle_buffer(int dev) {
-    static IdleBuffer idle[kPoolDevices];
-    return dev >= 0 && dev < kPoolDevices ? &idle[dev] : nullptr;
+lum::IdleBuffer* idle_buffer(int dev) {
+    static std::mutex mu;
+    static lum::IdleBuffer* idle[kPoolDevices] = {};   // never deleted: scenes may outlive this file's statics
+    if (dev < 0 || dev >= kPoolDevices) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!idle[dev]) idle[dev] = new lum::IdleBuffer([](void* p) { cudaFree(p); }, kPoolKeepBytes);
+    return idle[dev];
 }
 
 // What is kept for reuse goes back to the driver.
 void give_back_idle(int dev) {
     cudaMemPool_t pool = nullptr;
     if (scene_pool(dev, &pool) == LUM_OK) cudaMemPoolTrimTo(pool, 0);
-    if (IdleBuffer* idle = idle_buffer(dev)) {
-        std::lock_guard<std::mutex> lk(idle->mu);
-        if (idle->ptr) cudaFree(idle->ptr);
-        idle->ptr = nullptr;
-        idle->bytes = 0;
-    }
+    if (lum::IdleBuffer* idle = idle_buffer(dev)) idle->give_back();
 }
 
 // Pool allocation ordered on the scene's stream; `sync` waits for it, so that the memory can be
@@ -684,13 +679,12 @@ lum_status pool_alloc(lum_scene* s, void** ptr, size_t bytes, bool sync = true) 
     cudaMemPool_t pool = nullptr;
     lum_status st = scene_pool(s->device, &pool);
     if (st != LUM_OK) return st;
-    cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        give_back_idle(s->device);
-        e = cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream);
-    }
-    CU(e, "cudaMallocFromPoolAsync");
+    CU(lum::alloc_or_release(cudaErrorMemoryAllocation,
+                             [&] { return cudaMallocFromPoolAsync(ptr, bytes, pool, s->stream); },
+                             [&] {
+                                 cudaGetLastError();
+                                 give_back_idle(s->device);
+                             }), "cudaMallocFromPoolAsync");
     if (sync) CU(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
     return LUM_OK;
 }
@@ -1080,6 +1074,7 @@ lum_status lum_scene_create(const lum_scene_desc* desc, lum_scene** out) {
     };
     cudaError_t ce = cudaGetDevice(&s->device);
     if (ce != cudaSuccess) return cleanup(cuda_fail(ce, "cudaGetDevice"));
+    if ((s->idle = idle_buffer(s->device))) s->idle->add_owner();
     if ((ce = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess)
         return cleanup(cuda_fail(ce, "cudaStreamCreate"));
     if ((ce = cudaEventCreate(&s->ev0)) != cudaSuccess || (ce = cudaEventCreate(&s->ev1)) != cudaSuccess)
@@ -1196,6 +1191,7 @@ lum_status lum_scene_destroy(lum_scene* s) {
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->stream) cudaStreamDestroy(s->stream);
+    if (s->idle) s->idle->remove_owner();
     delete s;
     return LUM_OK;
 }
@@ -1283,7 +1279,7 @@ lum_status lum_scene_set_envmap(lum_scene* s, const float* rgb, uint32_t width, 
     s->dev.env_w = s->dev.env_h = 0;
     if (!rgb) return LUM_OK;
     const size_t bytes = sizeof(float) * 3 * (size_t)width * height;
-    CU(cudaMalloc(&s->d_env, bytes), "cudaMalloc");
+    CU(lum::device_malloc(s->device, &s->d_env, bytes), "cudaMalloc");
     CU(cudaMemcpy(s->d_env, rgb, bytes, cudaMemcpyHostToDevice), "cudaMemcpy H2D");
     s->dev.env = (const float*)s->d_env;
     s->dev.env_w = width;
@@ -1481,38 +1477,25 @@ lum_status prepare_render(lum_scene* s, const lum_render_params* params, SceneDe
     return LUM_OK;
 }
 
+cudaError_t device_malloc(int device, void** ptr, size_t bytes) {
+    return alloc_or_release(cudaErrorMemoryAllocation, [&] { return cudaMalloc(ptr, bytes); },
+                            [&] {
+                                cudaGetLastError();
+                                give_back_idle(device);
+                            });
+}
+
 lum_status scratch_alloc(lum_scene* s, void** ptr, size_t* bytes) {
-    if (IdleBuffer* idle = idle_buffer(s->device)) {
-        std::lock_guard<std::mutex> lk(idle->mu);
-        if (idle->ptr && idle->bytes >= *bytes) {
-            *ptr = idle->ptr;
-            *bytes = idle->bytes;
-            idle->ptr = nullptr;
-            idle->bytes = 0;
-            return LUM_OK;
-        }
-    }
-    cudaError_t e = cudaMalloc(ptr, *bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        give_back_idle(s->device);
-        e = cudaMalloc(ptr, *bytes);
-    }
-    CU(e, "cudaMalloc");
+    IdleBuffer* idle = idle_buffer(s->device);
+    if (idle && (*ptr = idle->take(bytes))) return LUM_OK;
+    CU(device_malloc(s->device, ptr, *bytes), "cudaMalloc");
     return LUM_OK;
 }
 
 void scratch_free(lum_scene* s, void* ptr, size_t bytes) {
     cudaStreamSynchronize(s->stream);   // a call that failed may have work in flight
-    IdleBuffer* idle = idle_buffer(s->device);
-    if (idle && bytes <= kPoolKeepBytes) {
-        std::lock_guard<std::mutex> lk(idle->mu);
-        if (bytes > idle->bytes) {
-            std::swap(ptr, idle->ptr);
-            idle->bytes = bytes;
-        }
-    }
-    if (ptr) cudaFree(ptr);
+    if (IdleBuffer* idle = idle_buffer(s->device)) idle->put(ptr, bytes);
+    else cudaFree(ptr);
 }
 
 int scene_max_material_kind(const lum_scene* s) { return s ? s->max_mat_kind : 0; }

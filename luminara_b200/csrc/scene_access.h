@@ -23,9 +23,12 @@ lum_status prepare_render(lum_scene* s, const lum_render_params* params, SceneDe
 lum_status scene_view(lum_scene* s, const lum_render_params* params, SceneDev& dev, RenderDev& R, int& device);
 // Largest LUM_MAT_* kind among the scene's materials (0 when it has none).
 int scene_max_material_kind(const lum_scene* s);
+// cudaMalloc on the current device `device`; when it finds no memory, what this library keeps for reuse
+// goes back to the driver first.
+cudaError_t device_malloc(int device, void** ptr, size_t bytes);
 // Device memory of one call, at least `*bytes` (set to its size).  scratch_free waits for the scene's
-// stream; the largest freed buffer (up to 4 GiB) is kept per device for the next call, and goes back
-// to the driver when an allocation finds no memory.
+// stream; the largest freed buffer (up to 4 GiB) is kept per device for the next call
+// (idle_buffer.h says when it goes back).
 lum_status scratch_alloc(lum_scene* s, void** ptr, size_t* bytes);
 void scratch_free(lum_scene* s, void* ptr, size_t bytes);
 // The mutex that serialises calls on one scene handle (held by every entry point that reads

@@ -783,7 +783,7 @@ lum_status create_batch(lum_scene* const* scenes, const lum_render_params* param
     if (e != cudaSuccess) return fail_out(wf_cuda(e, "cudaSetDevice"));
     if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreate(&b->ev0)) != cudaSuccess || (e = cudaEventCreate(&b->ev1)) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_mem, off)) != cudaSuccess ||
+        (e = lum::device_malloc(b->device, (void**)&b->d_mem, off)) != cudaSuccess ||
         (e = cudaHostAlloc((void**)&b->h_done, sizeof(uint32_t), cudaHostAllocDefault)) != cudaSuccess)
         return fail_out(wf_cuda(e, "batch allocation"));
     char* m = (char*)b->d_mem;
