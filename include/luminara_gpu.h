@@ -345,9 +345,11 @@ lum_status lum_scene_info(const lum_scene* scene, uint32_t* n_prims, uint32_t* n
 
 /* Replaces render::render (src/render.rs:1557-1731): renders into a caller-owned HOST
  * buffer of width*height*3 floats (crop size when has_crop).  Device output buffers are
- * owned by the scene.  The image is read back through pinned staging buffers shared per
- * device (4 MB chunks, copied into out_rgb by up to 8 host threads); a call that finds them
- * in use by another thread copies directly.  stats may be NULL. */
+ * owned by the scene.  An image of 8 MB or more, or of 1 MB or more when renders follow one
+ * another within 2 ms, is read back through two pinned staging buffers shared per device (chunks of
+ * up to 8 MB, copied into out_rgb by up to 16 host threads, by more than 8 only as far as
+ * OMP_NUM_THREADS allows); a call that finds them in use by another thread copies directly.
+ * stats may be NULL. */
 lum_status lum_render(lum_scene* scene, const lum_render_params* params, float* out_rgb,
                       lum_stats* stats);
 

@@ -10,6 +10,7 @@
 #include <omp.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -27,6 +28,7 @@
 #include "idle_buffer.h"
 #include "kernels.h"
 #include "scene_access.h"
+#include "staging_rule.h"
 
 namespace {
 
@@ -708,128 +710,173 @@ lum_status ensure(lum_scene* s, void** ptr, size_t* cap, size_t bytes) {
 // Transfers between pageable host memory and the device through two pinned staging chunks: the
 // copy engine moves one chunk while host threads copy the other.  A direct cudaMemcpy into
 // pageable memory took 1.4-6.3 ms for a 25 MB frame on the B200 box, a copy into pinned memory
-// 0.46 ms.  A million rays up and their hits down (88 MB) 14.1 -> 4.5 ms with 8 MB chunks and 16
-// threads (4 MB and 8 threads 5.7), full HD AOVs (21 MB) 1.66 -> 1.04 ms with 2 MB and 4.  The staging buffers are per device and shared; a call that finds them busy (another
-// thread's) copies directly, as do transfers below kStageMin, where the driver's own path is
-// as fast.
-constexpr size_t kStageChunk = 8u << 20;
-constexpr size_t kStageMin = 1u << 20;
+// 0.46 ms.  Transfers up to kStageLong take chunks of up to 4 MB and 4 threads, longer ones 8 MB and
+// 16 threads, which they alone gain from: sleeping threads are woken for each call.  A million rays (46
+// MB up, their hits 46 MB down) 12.6 -> 3.8 ms (4 MB chunks 4.5); 400k rays with 4 / 8 / 16 threads right
+// after another call 1.6 / 1.7 / 1.8 ms, with the threads asleep 2.0 / 2.8 / 3.5; 1080p frames 1.2 / 1.3 /
+// 1.25 and 1.25 / 1.65 / 1.9.  The staging buffers are per device and shared; staging_rule.h says
+// which calls take them.  A transfer that finds them busy (another thread's) copies directly.
+constexpr size_t kStageLong = 32u << 20;
+constexpr size_t kStageMin = lum::StagingRule::kMin;   // shorter transfers of any call: the driver's own path is as fast
+size_t stage_chunk(size_t bytes) { return bytes > kStageLong ? (size_t)8 << 20 : (size_t)4 << 20; }
 
 struct Staging {
-    std::mutex mu;
+    std::mutex mu;                            // of the buffers
     unsigned char* buf[2] = {nullptr, nullptr};
-    cudaEvent_t ev[2] = {nullptr, nullptr};
+    cudaEvent_t ev[2] = {nullptr, nullptr};   // recorded after a buffer's last copy, on any stream
+    std::atomic<size_t> size{0};              // of each buffer; 0: not allocated
+    std::mutex rule_mu;
+    lum::StagingRule rule;
 };
 
-Staging* staging(int dev) {
-    static Staging st[kPoolDevices];
-    return dev >= 0 && dev < kPoolDevices ? &st[dev] : nullptr;
+// Frames have buffers apart from ray sets and AOVs: a thread that sends one ray set after another does
+// not push another thread's frames to the direct copy (1080p frames 1.3 ms alone, 3.0-3.4 ms then).
+Staging* staging(int dev, lum::StagingUse use) {
+    static Staging st[kPoolDevices][2];
+    return dev >= 0 && dev < kPoolDevices ? &st[dev][use == lum::StagingUse::Frame ? 0 : 1] : nullptr;
 }
 
-// Two team sizes only: libgomp rebuilds its team when the size changes.
-void host_copy(unsigned char* dst, const unsigned char* src, size_t n) {
-    const int nt = std::max(1, std::min(n > (3u << 20) ? 16 : 4, omp_get_num_procs()));
-    const size_t slice = (n / nt + 4095) & ~(size_t)4095;
-#pragma omp parallel for num_threads(nt) schedule(static)
-    for (int k = 0; k < nt; ++k) {
+void host_copy(unsigned char* dst, const unsigned char* src, size_t n, int threads) {
+    const size_t slice = (n / threads + 4095) & ~(size_t)4095;
+#pragma omp parallel for num_threads(threads) schedule(static)
+    for (int k = 0; k < threads; ++k) {
         const size_t o = (size_t)k * slice;
-        if (o < n) std::memcpy(dst + o, src + o, k == nt - 1 ? n - o : std::min(slice, n - o));
+        if (o < n) std::memcpy(dst + o, src + o, k == threads - 1 ? n - o : std::min(slice, n - o));
     }
 }
 
-// One call's transfers on one stream: holds the staging buffers (if they are free) until the call
-// ends, with no copy of theirs in flight.
+// One call's transfers on one stream, `bytes` the largest of them (of planes: all).  Each holds the
+// staging buffers, if they are free, until the host has no more to do with them; a copy
+// that is still in flight then is waited for by the buffers' next user, through their events.
 class Transfers {
 public:
-    Transfers(int device, cudaStream_t stream) : stream_(stream), sg_(staging(device)) {
-        if (sg_) lk_ = std::unique_lock<std::mutex>(sg_->mu, std::try_to_lock);
-        if (!lk_.owns_lock()) sg_ = nullptr;
+    Transfers(int device, cudaStream_t stream, lum::StagingUse use, size_t bytes)
+        : stream_(stream), sg_(staging(device, use)), bytes_(bytes) {
+        if (!sg_) return;
+        std::lock_guard<std::mutex> lk(sg_->rule_mu);
+        staged_ = sg_->rule.begin(use, bytes, sg_->size >= stage_chunk(bytes), now());
     }
     ~Transfers() {
-        if (pending_) cudaStreamSynchronize(stream_);   // before another call writes the buffers
+        if (!sg_) return;
+        std::lock_guard<std::mutex> lk(sg_->rule_mu);
+        sg_->rule.end(bytes_, now());
     }
 
     // host -> device; the source may be reused on return.
     lum_status up(void* dst, const void* src, size_t bytes) {
-        if (!staged(bytes)) {
+        Hold hold(*this, bytes);
+        if (!hold.lk) {
             CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream_), "cudaMemcpyAsync H2D");
             return LUM_OK;
         }
-        lum_status st = prepare();
-        if (st != LUM_OK) return st;
         const size_t chunk = chunk_of(bytes);
         for (size_t o = 0; o < bytes; o += chunk) {
             const size_t n = std::min(chunk, bytes - o);
             const int b = next();
             CU(cudaEventSynchronize(sg_->ev[b]), "H2D");   // the buffer's last copy has left it
-            host_copy(sg_->buf[b], static_cast<const unsigned char*>(src) + o, n);
+            host_copy(sg_->buf[b], static_cast<const unsigned char*>(src) + o, n, threads_of(bytes));
+            hold.pending = true;
             CU(cudaMemcpyAsync(static_cast<unsigned char*>(dst) + o, sg_->buf[b], n, cudaMemcpyHostToDevice, stream_),
                "cudaMemcpyAsync H2D");
             CU(cudaEventRecord(sg_->ev[b], stream_), "cudaEventRecord");
-            pending_ = true;
+            hold.pending = false;
         }
         return LUM_OK;
     }
 
     // device -> host, waited for.
     lum_status down(void* dst, const void* src, size_t bytes) {
-        if (!staged(bytes)) {
+        Hold hold(*this, bytes);
+        if (!hold.lk) {
             CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_), "cudaMemcpyAsync D2H");
             CU(cudaStreamSynchronize(stream_), "D2H");
-            pending_ = false;
             return LUM_OK;
         }
-        lum_status st = prepare();
-        if (st != LUM_OK) return st;
         const size_t chunk = chunk_of(bytes);
         unsigned char *d = static_cast<unsigned char*>(dst), *last_dst = nullptr;
         int last_b = 0;
         size_t last_n = 0;
+        hold.pending = true;
         for (size_t o = 0;; o += chunk) {
             const bool more = o < bytes;
             const int b = more ? next() : 0;
             const size_t n = more ? std::min(chunk, bytes - o) : 0;
-            if (more) {   // into the buffer whose previous chunk the host has copied out
+            if (more) {   // into the buffer whose previous chunk the host or another stream has copied out
+                CU(cudaStreamWaitEvent(stream_, sg_->ev[b], 0), "cudaStreamWaitEvent");
                 CU(cudaMemcpyAsync(sg_->buf[b], static_cast<const unsigned char*>(src) + o, n, cudaMemcpyDeviceToHost,
                                    stream_), "cudaMemcpyAsync D2H");
                 CU(cudaEventRecord(sg_->ev[b], stream_), "cudaEventRecord");
-                pending_ = true;
             }
             if (last_n) {   // the chunk before it to its place
                 CU(cudaEventSynchronize(sg_->ev[last_b]), "D2H");
-                host_copy(last_dst, sg_->buf[last_b], last_n);
+                host_copy(last_dst, sg_->buf[last_b], last_n, threads_of(bytes));
             }
             if (!more) break;
             last_dst = d + o;
             last_b = b;
             last_n = n;
         }
-        pending_ = false;
+        hold.pending = false;
         return LUM_OK;
     }
 
 private:
-    bool staged(size_t bytes) const { return sg_ && bytes >= kStageMin; }
+    // The staging buffers for one transfer; empty (lk unlocked) if it copies directly.
+    struct Hold {
+        Hold(Transfers& t, size_t bytes) : stream(t.stream_) {
+            if (!t.staged_ || bytes < kStageMin) return;
+            lk = std::unique_lock<std::mutex>(t.sg_->mu, std::try_to_lock);
+            if (lk && !prepare(*t.sg_, stage_chunk(bytes))) lk.unlock();
+        }
+        ~Hold() {
+            if (pending) cudaStreamSynchronize(stream);   // a transfer that failed, before another uses the buffers
+        }
+        cudaStream_t stream;
+        bool pending = false;   // a copy through the buffers without an event behind it
+        std::unique_lock<std::mutex> lk;
+    };
+    static bool prepare(Staging& sg, size_t size) {   // false: no pinned memory
+        bool ok = true;
+        for (int b = 0; b < 2; ++b)
+            ok = ok && (sg.ev[b] || cudaEventCreateWithFlags(&sg.ev[b], cudaEventDisableTiming) == cudaSuccess);
+        if (ok && sg.size < size) {
+            sg.size = 0;
+            for (int b = 0; b < 2; ++b) {
+                if (sg.buf[b]) {
+                    cudaEventSynchronize(sg.ev[b]);   // its last copy has left it
+                    cudaFreeHost(sg.buf[b]);
+                }
+                sg.buf[b] = nullptr;
+                ok = ok && cudaHostAlloc((void**)&sg.buf[b], size, cudaHostAllocPortable) == cudaSuccess;
+            }
+            if (ok) sg.size = size;
+        }
+        if (!ok) cudaGetLastError();
+        return ok;
+    }
     static size_t chunk_of(size_t bytes) {   // at least four chunks of a short transfer overlap
-        return std::min(kStageChunk, std::max((size_t)256 << 10, (bytes / 4 + 4095) & ~(size_t)4095));
+        return std::min(stage_chunk(bytes), std::max((size_t)256 << 10, (bytes / 4 + 4095) & ~(size_t)4095));
+    }
+    // One team for all chunks of a transfer, of two sizes only: libgomp rebuilds its team when the size
+    // changes.  Above 8 threads only as far as OMP_NUM_THREADS goes.
+    static int threads_of(size_t bytes) {
+        const int most = std::min(omp_get_num_procs(), std::max(8, omp_get_max_threads()));
+        return std::max(1, std::min(bytes > kStageLong ? 16 : 4, most));
+    }
+    static int64_t now() {
+        return std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch())
+            .count();
     }
     int next() { return turn_ ^= 1; }
-    lum_status prepare() {
-        for (int b = 0; b < 2; ++b) {
-            if (!sg_->buf[b]) CU(cudaHostAlloc((void**)&sg_->buf[b], kStageChunk, cudaHostAllocPortable), "cudaHostAlloc");
-            if (!sg_->ev[b]) CU(cudaEventCreateWithFlags(&sg_->ev[b], cudaEventDisableTiming), "cudaEventCreate");
-        }
-        return LUM_OK;
-    }
     cudaStream_t stream_;
     Staging* sg_;
-    std::unique_lock<std::mutex> lk_;
+    size_t bytes_;
+    bool staged_ = false;
     int turn_ = 0;
-    bool pending_ = false;   // copies through the buffers not known to have finished
 };
 
 lum_status readback(lum_scene* s, void* dst, const void* src, size_t bytes, cudaStream_t stream) {
-    return Transfers(s->device, stream).down(dst, src, bytes);
+    return Transfers(s->device, stream, lum::StagingUse::Frame, bytes).down(dst, src, bytes);
 }
 
 lum_status make_render_dev(const lum_scene* s, const lum_render_params& p, lum::RenderDev& R) {
@@ -1309,7 +1356,7 @@ lum_status lum_render_aov(lum_scene* s, const lum_render_params* params, float* 
                        s->d_work, s->stream), "aov launch");
     lum::WorkCounters wc{};
     CU(cudaMemcpyAsync(&wc, s->d_work, sizeof wc, cudaMemcpyDeviceToHost, s->stream), "D2H");
-    Transfers tr(s->device, s->stream);
+    Transfers tr(s->device, s->stream, lum::StagingUse::Planes, 10 * px);   // after the copy above, which has waited for the kernel
     if (depth) st = tr.down(depth, d_depth, 4 * px);
     if (st == LUM_OK && normals) st = tr.down(normals, d_norm, 3 * px);
     if (st == LUM_OK && albedo) st = tr.down(albedo, d_alb, 3 * px);
@@ -1422,7 +1469,7 @@ lum_status lum_intersect(lum_scene* s, const lum_ray* rays, uint32_t n, lum_hit*
     if (st != LUM_OK) return st;
     lum_ray* d_r = (lum_ray*)s->d_rays;
     lum_hit* d_h = (lum_hit*)((char*)s->d_rays + rb);
-    Transfers tr(s->device, s->stream);
+    Transfers tr(s->device, s->stream, lum::StagingUse::Rays, sizeof(lum_ray) * (size_t)n);
     if ((st = tr.up(d_r, rays, sizeof(lum_ray) * (size_t)n)) != LUM_OK) return st;
     CU(cudaMemsetAsync(s->d_work, 0, sizeof(lum::WorkCounters), s->stream), "memset");
     CU(lum::launch_intersect(s->dev, d_r, n, d_h, s->d_work, s->stream), "intersect launch");
@@ -1443,7 +1490,7 @@ lum_status lum_occluded(lum_scene* s, const lum_ray* rays, uint32_t n, int32_t* 
     if (st != LUM_OK) return st;
     lum_ray* d_r = (lum_ray*)s->d_rays;
     int32_t* d_o = (int32_t*)((char*)s->d_rays + rb);
-    Transfers tr(s->device, s->stream);
+    Transfers tr(s->device, s->stream, lum::StagingUse::Rays, sizeof(lum_ray) * (size_t)n);
     if ((st = tr.up(d_r, rays, sizeof(lum_ray) * (size_t)n)) != LUM_OK) return st;
     CU(cudaMemsetAsync(s->d_work, 0, sizeof(lum::WorkCounters), s->stream), "memset");
     CU(lum::launch_occluded(s->dev, d_r, n, d_o, s->d_work, s->stream), "occluded launch");
