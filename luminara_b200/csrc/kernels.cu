@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -365,6 +366,34 @@ size_t render_scratch_bytes(const RenderDev& R, const RenderGroups& g) {
 // fixed-point sums there (zeroed first) and writes no pixels.  Otherwise split tiles need
 // `scratch` (render_scratch_bytes); only as many tiles are split as its `scratch_bytes` hold,
 // the others are rendered whole.
+using RenderFn = void (*)(SceneDev, RenderDev, float*, WorkCounters*, TaskPlan);
+
+// The build of a scene and render: scenes without the other materials and backgrounds, without
+// lights, or made of spheres with the basic materials run builds without the code they cannot
+// reach; the counter build is the general one: the same paths either way.
+template <bool COUNT>
+static RenderFn render_kernel(const SceneDev& S, const RenderDev& R) {
+    auto build = [&](auto ext, auto sph, auto cls) -> RenderFn {
+        constexpr bool E = decltype(ext)::value, P = decltype(sph)::value;
+        constexpr int C = decltype(cls)::value;
+        return COUNT || S.n_lights > 0 ? k_render<COUNT, E, true, P, C> : k_render<COUNT, E, COUNT, P, C>;
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    if (R.ext && S.n_big > 0) return build(Yes(), No(), std::integral_constant<int, CLS_GROUND>());
+    if (R.ext) return build(Yes(), No(), std::integral_constant<int, CLS_ALL>());
+    if constexpr (!COUNT) {
+        if (S.spheres_basic) return build(No(), Yes(), std::integral_constant<int, CLS_ALL>());
+        const bool many = S.n_prims >= many_prims(S.cls);
+        if (S.cls == CLS_QUAD && many) return build(No(), No(), std::integral_constant<int, CLS_QUAD_MANY>());
+        if (S.cls == CLS_QUAD) return build(No(), No(), std::integral_constant<int, CLS_QUAD>());
+        if (S.cls == CLS_MESH && many) return build(No(), No(), std::integral_constant<int, CLS_MESH_MANY>());
+        if (S.cls == CLS_MESH) return build(No(), No(), std::integral_constant<int, CLS_MESH>());
+        if (many) return build(No(), No(), std::integral_constant<int, CLS_MANY>());
+    }
+    return build(No(), No(), std::integral_constant<int, CLS_ALL>());
+}
+
 template <bool COUNT>
 static cudaError_t launch_render_t(const SceneDev& S, const RenderDev& R, float* out, WorkCounters* wc,
                                    cudaStream_t stream, int blocks_per_sm, RenderGroups grp, void* scratch,
@@ -399,34 +428,13 @@ static cudaError_t launch_render_t(const SceneDev& S, const RenderDev& R, float*
         cudaError_t e = cudaMemsetAsync(pix_sums, 0, 32 * (size_t)R.w * R.h, stream);
         if (e != cudaSuccess) return e;
     }
-    const bool nee = COUNT || S.n_lights > 0;
-    const bool sph = !COUNT && !R.ext && S.spheres_basic;
-    const int cls = (COUNT || R.ext || sph) ? (int)CLS_ALL : S.cls;
-    const bool many = !COUNT && S.n_prims >= many_prims(cls);
-    auto kernel = R.ext && S.n_big > 0 ? (nee ? k_render<COUNT, true, true, false, CLS_GROUND>
-                                              : k_render<COUNT, true, COUNT, false, CLS_GROUND>)
-                : R.ext ? (nee ? k_render<COUNT, true, true, false> : k_render<COUNT, true, COUNT, false>)
-                : sph   ? (nee ? k_render<COUNT, false, true, !COUNT> : k_render<COUNT, false, COUNT, !COUNT>)
-                : cls == CLS_QUAD && many ? (nee ? k_render<COUNT, false, true, false, CLS_QUAD_MANY>
-                                                 : k_render<COUNT, false, COUNT, false, CLS_QUAD_MANY>)
-                : cls == CLS_QUAD ? (nee ? k_render<COUNT, false, true, false, CLS_QUAD>
-                                         : k_render<COUNT, false, COUNT, false, CLS_QUAD>)
-                : cls == CLS_MESH && many ? (nee ? k_render<COUNT, false, true, false, CLS_MESH_MANY>
-                                                 : k_render<COUNT, false, COUNT, false, CLS_MESH_MANY>)
-                : cls == CLS_MESH ? (nee ? k_render<COUNT, false, true, false, CLS_MESH>
-                                         : k_render<COUNT, false, COUNT, false, CLS_MESH>)
-                : many ? (nee ? k_render<COUNT, false, true, false, CLS_MANY>
-                              : k_render<COUNT, false, COUNT, false, CLS_MANY>)
-                       : (nee ? k_render<COUNT, false, true, false> : k_render<COUNT, false, COUNT, false>);
+    const RenderFn kernel = render_kernel<COUNT>(S, R);
     // the traversal stack sized to the scene's BVH; resident blocks for that size
     const size_t smem = stack_smem(S.stack_depth, kRenderThreads);
     if (blocks_per_sm == occ) blocks_per_sm = kernel_occupancy((const void*)kernel, smem);
     int grid = num_sms() * blocks_per_sm;
     int blocks_needed = (int)((n_total + 3) / 4);   // 4 warps per block, one task per warp at least
     if (grid > blocks_needed) grid = blocks_needed > 0 ? blocks_needed : 1;
-    // (kernel above: scenes without the other materials and backgrounds, without lights, or
-    // made of spheres with the basic materials run builds without the code they cannot reach;
-    // the counter build is the general one: the same paths either way)
     kernel<<<grid, kRenderThreads, smem, stream>>>(S, R, out, wc, TP);
     cudaError_t e = cudaGetLastError();
     const uint32_t n_split = n_tiles - TP.n_whole;

@@ -388,9 +388,7 @@ __device__ __forceinline__ bool test_prim(const SceneDev& S, int i, const Ray& r
         }
         default: {
             if constexpr (!cls_has_prim<CLS>(PT_FOG_BOX)) return false;
-            const bool fog_hit = !cls_is_quad<CLS>() ? hit_fog_cold(type, a, b, c, ray, tmin, hit.t, t)
-                                                 : hit_fog(type, a, b, c, ray, tmin, hit.t, t);
-            if (fog_hit) { hit.t = t; hit.prim = i; return true; }
+            if (hit_fog_cold(type, a, b, c, ray, tmin, hit.t, t)) { hit.t = t; hit.prim = i; return true; }
             return false;
         }
     }
@@ -820,8 +818,7 @@ struct ScatterMore {
     V dir, att, org;
     bool ok;
 };
-__device__ __forceinline__ ScatterMore scatter_more(
-const MatDev* mp, V rd, V hp, V hn, float4 s, uint32_t key0,
+__device__ __forceinline__ ScatterMore scatter_more(const MatDev* mp, V rd, V hp, V hn, float4 s, uint32_t key0,
                                                        uint32_t key1, uint32_t pixel, uint32_t stratum,
                                                        uint32_t bounce) {
     const MatDev& m = *mp;
