@@ -175,3 +175,64 @@ def test_aov_builds_at_ragged_sizes_match_the_oracle(build, size):
     assert (np.abs(got[0] - want[0])[hit] <= 5e-4 * want[0][hit]).mean() >= 0.98
     assert (np.abs(got[1].astype(int) - want[1].astype(int)) <= 1).mean() >= 0.98
     assert (np.abs(got[2].astype(int) - want[2].astype(int)) <= 1).mean() >= 0.96
+
+
+@pytest.mark.parametrize("build", ["spheres", "box_room", "zoo"])
+def test_aov_crops_equal_the_frame(build):
+    """AOVs of crops with one live lane, a row, a column and partial tiles, against the whole frame's.  A
+    1x1 frame's ray has no finite direction (its pixel grid has no width), so it meets nothing."""
+    world, cfg = (W.random_spheres if build == "spheres" else SCENES[build][0])(*((64, 48) if build == "spheres" else ()))
+    sc = L.GpuScene(world)
+    frame = sc.render_aov(cfg)
+    assert all(p.any() for p in frame)
+    for crop in ((0, 0, 1, 1), (33, 20, 1, 1), (40, 30, 1, 9), (5, 47, 17, 1), (7, 3, 9, 5), (40, 30, 24, 18)):
+        cfg.crop = crop
+        x, y, w, h = crop
+        for part, whole in zip(sc.render_aov(cfg), frame):
+            np.testing.assert_array_equal(part, whole[y:y + h, x:x + w])
+    cfg.crop = None
+    cfg.width = cfg.height = 1
+    assert not any(p.any() for p in sc.render_aov(cfg))
+    sc.close()
+
+
+def _sampled_scene(build):
+    if build == "quads":
+        return W.diff_quads(64, 48, 20, n_quads=40)
+    if build == "spheres":
+        return W.random_spheres(64, 48, 20)
+    if build == "mixed":
+        return W.uneven_scene(np.random.default_rng(1), 300, 64, 48, 20)
+    return SCENES[build][0]()
+
+
+SAMPLED = ["spheres", "box_room", "quads", "mesh", "zoo", "mixed"]
+
+
+@pytest.mark.parametrize("threshold", [0.0, 0.05])
+@pytest.mark.parametrize("build", SAMPLED)
+def test_adaptive_crops_equal_the_frame(build, threshold):
+    """Every build of the adaptive kernel, bit for bit: a pixel's samples and its stop do not depend on the
+    pixels that share its pool, so crops with 1 to 32 pixels per tile equal the whole frame.  25 strata
+    in rounds of 16 and 9."""
+    world, cfg = _sampled_scene(build)
+    cfg.samples_per_pixel, cfg.adaptive, cfg.adaptive_threshold = 20, True, threshold
+    sc = L.GpuScene(world)
+    frame, st = sc.render(cfg)
+    assert (st.paths == 25 * 64 * 48) == (threshold == 0.0) and st.paths >= 16 * 64 * 48
+    for x, y, w, h in ((0, 0, 1, 1), (33, 20, 1, 1), (7, 3, 9, 5), (50, 41, 7, 4), (11, 30, 3, 18), (0, 5, 64, 3)):
+        cfg.crop = (x, y, w, h)
+        np.testing.assert_array_equal(sc.render(cfg)[0], frame[y:y + h, x:x + w])
+    sc.close()
+
+
+@pytest.mark.parametrize("build", SAMPLED)
+def test_time_limit_that_does_not_run_out_equals_the_render(build):
+    """Every time-limited build, its pool one tile's strata, gives the plain render's sums."""
+    world, cfg = _sampled_scene(build)
+    cfg.width, cfg.height, cfg.samples_per_pixel = 37, 21, 20
+    sc = L.GpuScene(world)
+    plain, _ = sc.render(cfg)
+    cfg.time_limit = 1000.0
+    np.testing.assert_array_equal(sc.render(cfg)[0], plain)
+    sc.close()
