@@ -1057,7 +1057,8 @@ lum_status lum_scene_create(const lum_scene_desc* desc, lum_scene** out) {
     for (uint32_t i = 0; i < desc->n_materials && sph; ++i)
         sph = desc->materials[i].kind >= LUM_MAT_LAMBERTIAN && desc->materials[i].kind <= LUM_MAT_EMISSIVE;
     // its big spheres (grounds: radius from kBigSphere up, a few at most) stay out of the BVH; every
-    // walk tests them first (walk_warp).  Closest hits do not depend on the order of the tests.
+    // walk tests them first (walk_warp).  Closest hits depend on the order of the tests only where two are
+    // exactly as far: the one tested last wins, so a big sphere gives way to a small one there.
     std::vector<uint32_t> in_tree, big;
     for (size_t k = 0; k < F.prims.size(); ++k)
         (sph && F.prims[k].rec[3] >= lum::kBigSphere ? big : in_tree).push_back((uint32_t)k);
@@ -1356,7 +1357,7 @@ lum_status lum_render_aov(lum_scene* s, const lum_render_params* params, float* 
                        s->d_work, s->stream), "aov launch");
     lum::WorkCounters wc{};
     CU(cudaMemcpyAsync(&wc, s->d_work, sizeof wc, cudaMemcpyDeviceToHost, s->stream), "D2H");
-    Transfers tr(s->device, s->stream, lum::StagingUse::Planes, 10 * px);   // after the copy above, which has waited for the kernel
+    Transfers tr(s->device, s->stream, lum::StagingUse::Planes, 10 * px);   // the copy above has waited for the kernel
     if (depth) st = tr.down(depth, d_depth, 4 * px);
     if (st == LUM_OK && normals) st = tr.down(normals, d_norm, 3 * px);
     if (st == LUM_OK && albedo) st = tr.down(albedo, d_alb, 3 * px);

@@ -25,7 +25,9 @@ namespace lum {
 
 constexpr int kRenderThreads = 128;
 // Minimum resident blocks per SM requested from the register allocator: 7 (72 registers).  More warps
-// to hide the dependent node and primitive fetches outweigh the spills (40-130 bytes) up to there.
+// to hide the dependent node and primitive fetches outweigh the spills up to there (bytes of spill
+// stores with lights / without: other materials 218 / 108, with big spheres 186 / 112, general 150 / 104,
+// meshes 70 / 68, quads 60 / 0, spheres none).
 // On B200 with warp-convergent walks and the rare code out of line: general build (twelve mixed
 // scenes) 6 / 7 / 8 blocks 150.2 / 145.4 / 147.8 ms, other materials 7 / 8 / 9 10.8 / 11.0 / 10.9; classes 6
 // / 7 / 8 blocks: dense mesh 17.2 / 16.7 / 16.7 ms, quads 7.70 / 7.60 / 7.69, box room 1.64 / 1.63 /

@@ -111,7 +111,8 @@ __device__ __forceinline__ void sample_pool(const SceneDev& S, const RenderDev& 
     }
 }
 
-// a / n with r = 1 / n, correctly rounded (tracer.cuh's div_by in f64).
+// a / n with r = 1 / n (tracer.cuh's div_by in f64: no difference from the division in 2^30 draws with n
+// up to 2^27).
 __device__ __forceinline__ double div_by(double a, double n, double r) {
     const double q = a * r;
     return fma(fma(-q, n, a), r, q);

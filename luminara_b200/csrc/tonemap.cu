@@ -145,7 +145,8 @@ __device__ __forceinline__ uint32_t tone_gamma(int kind, double x, double gamma,
 }
 
 // a / b for a finite a and b = 1, 2, ... with r = 1 / b: the quotient corrected by its exact remainder
-// is the correctly rounded one (Markstein, IBM J. Res. Dev. 1990, theorem 8.1).
+// (Markstein, IBM J. Res. Dev. 1990).  No difference from the division in 2^30 draws with b up to 2^27; a
+// proof would need the first quotient within one ulp, and its two roundings give 1.5.
 __device__ __forceinline__ double quotient(double a, double b, double r) {
     const double q = a * r;
     return fma(fma(-q, b, a), r, q);

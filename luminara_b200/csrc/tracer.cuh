@@ -1305,9 +1305,11 @@ __device__ __forceinline__ unsigned long long globaltimer() {
 }
 
 // a / b for a finite a and b = 1, 2, ... with r = 1 / b rounded to nearest: the quotient a * r
-// corrected by its exact remainder, which is the correctly rounded quotient (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
-// 1990, theorem 8.1).  r = 0 stands for b = 0: the plain division.
+// corrected by its exact remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 1990).  His theorem 8.1 asks for a first quotient within one
+// ulp, and two roundings only give 1.5, so that this is the rounded quotient is checked, not proven:
+// no difference for any b below 2^16 and any mantissa of a, nor in 2^30 draws with b up to 2^24.
+// r = 0 stands for b = 0: the plain division.
 __device__ __forceinline__ float div_by(float a, float b, float r) {
     if (r == 0.0f) return a / b;
     const float q = a * r;
