@@ -296,15 +296,17 @@ enum : int {
 };
 // From these sizes a walk is long enough that the last lanes' search for a leaf costs the others more
 // than turning to the leaves early does.  Never against always, ms on B200:
-//   mixed primitives, 512x512 16 spp: 1,000 3.25 / 3.31, 2,000 4.10 / 4.13, 4,000 4.97 / 4.89 and 4.68 /
-//     4.49, 8,000 5.38 / 5.16, 16,000 6.10 / 5.71; 128x128: 1,000 0.49 / 0.50, 2,000 0.58 / 0.60, 4,000 0.70 / 0.68
+//   mixed primitives, 512x512 16 spp: 2,000 4.10 / 4.13, 4,000 4.97 / 4.89 and 4.68 / 4.49, 8,000 5.38 /
+//     5.16, 16,000 6.10 / 5.71; 128x128: 2,000 0.58 / 0.60, 4,000 0.70 / 0.68.  But a batch's scenes run side by
+//     side, and two builds at once cost more than that: batches of up to 16,000 primitives with the line at
+//     16,384 / 4,096 7.67 / 8.16, 16.5 / 17.1, 45.0 / 45.4
 //   quads, 512x512 64 spp: 128 2.11 / 2.12, 200 3.01 / 2.98, 300 3.92 / 3.82, 512 5.42 / 5.26, 1,000 7.21 /
 //     7.03; 256x256 16 spp, where the longest tasks count: 128 0.240 / 0.256, 300 0.424 / 0.432, 512 0.574 /
 //     0.578, 1,000 0.808 / 0.803
 //   meshes, 960x540 16 spp: 1,280 triangles 3.17 / 3.25, 20,480 4.03 / 4.04, 81,920 4.57 / 4.45, 327,680 5.25 / 4.90
 // Four lanes gave 2% less on the mesh; ratios of waiting to searching lanes (4, 8, 14) no more.
 __host__ constexpr int many_prims(int cls) {
-    return cls == CLS_MESH ? 65536 : cls == CLS_QUAD ? 512 : 4096;
+    return cls == CLS_MESH ? 65536 : cls == CLS_QUAD ? 512 : 16384;
 }
 template <int CLS>
 __host__ __device__ constexpr bool cls_is_quad() { return CLS == CLS_QUAD || CLS == CLS_QUAD_MANY; }
