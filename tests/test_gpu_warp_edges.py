@@ -180,7 +180,7 @@ def test_aov_builds_at_ragged_sizes_match_the_oracle(build, size):
 @pytest.mark.parametrize("n", [507, 508, 1000])
 def test_quad_builds_equal_the_other_modes(n):
     """Quad scenes of both sides of 512 quads (four are the lights), from which warps turn to the leaves
-    early: the batch's kernels, which never do, give the same image."""
+    early: the wavefront and the batched megakernel, which never do, give the same image."""
     from luminara_b200 import abi
     world, cfg = W.diff_quads(61, 35, 4, n_quads=n)
     sc = L.GpuScene(world)
